@@ -26,7 +26,8 @@ LIB = os.path.join(HERE, "lib")
 OBJ = os.path.join(HERE, "lib", "obj")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVCC_FLAGS = ARCH + ["-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
+# --split-compile=0: the optimiser works on a file's kernels in parallel
+NVCC_FLAGS = ARCH + ["--split-compile=0", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
                      "--expt-relaxed-constexpr", "-I" + os.path.join(ROOT, "include")]
 CC_FLAGS = ["-O3", "-fPIC", "-std=gnu11", "-fopenmp",
             "-I" + os.path.join(ROOT, "include")]

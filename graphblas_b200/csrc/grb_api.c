@@ -1126,6 +1126,18 @@ static GrB_Info write_back(GrB_Matrix C, grb_b200_dmatrix T, GrB_Matrix M,
     }
     GrB_Info info = to_dev(C);
     if (info == GrB_SUCCESS && M) info = to_dev(M);
+    // C<M> = T over a C that lies in M already: C becomes T.  Only a plain
+    // structural mask: under a valued one M's false entries are outside too.
+    if (info == GrB_SUCCESS && !accum && M && mask_applied && !f.comp && f.strct && !f.replace)
+    {
+        const int taken = grb_b200_dtake_masked(C->dev, T, M->dev);
+        if (taken != 1)
+        {
+            grb_b200_dmatrix_free(&T);
+            if (taken == 0) host_free(C);
+            return (GrB_Info)taken;
+        }
+    }
     if (info == GrB_SUCCESS)
         info = (GrB_Info)grb_b200_daccum_mask(C->dev, T, M ? M->dev : NULL, f.comp,
                                               f.strct, f.replace,

@@ -255,6 +255,37 @@ __device__ __forceinline__ I warp_last_le(const T *__restrict__ a, I n, T key, i
     return lo;
 }
 
+// The row of each lane's entry e (the lanes' entries ascend and lie before
+// P[nrows], and row r0 starts at or before the first): the largest r with
+// P[r] <= e.  The warp reads the next 32 row starts at once and every lane
+// searches them by shuffles, so that 32 entries of many short or empty rows
+// take one load and six shuffles, where a walk takes a dependent load a row.
+// All lanes call it; one past the end of its entries passes the last of them.
+template <typename P_t, typename E_t>
+__device__ __forceinline__ E_t warp_rows(const P_t *__restrict__ P, E_t nrows, E_t r0, E_t e,
+                                         int lane)
+{
+    E_t r = r0;
+    bool done = false;
+    while (true) {
+        const E_t c = r0 + 1 + lane;
+        const P_t v = P[c < nrows ? c : nrows];
+        int cnt = 0;
+        #pragma unroll
+        for (int step = 16; step > 0; step >>= 1) {
+            const P_t t = __shfl_sync(0xffffffffu, v, cnt + step - 1);
+            if (t <= (P_t)e) cnt += step;
+        }
+        const P_t last = __shfl_sync(0xffffffffu, v, 31);     // by every lane
+        const bool more = cnt == 31 && last <= (P_t)e;
+        const bool go = more && !done;
+        if (!done) r = r0 + cnt + (more ? 1 : 0);
+        done |= !more;
+        if (!__any_sync(0xffffffffu, go)) return r;
+        r0 += 32;
+    }
+}
+
 // first position p in [lo,hi) with a[p] > key
 __device__ __forceinline__ int32_t upper_bound(const int32_t *a, int32_t lo,
                                                int32_t hi, int32_t key)

@@ -116,11 +116,11 @@ k_dot3_classify(const int32_t *__restrict__ Mp, const int32_t *__restrict__ Mj,
         const int64_t pm = base + lane;
         const bool valid = pm < mnz;
         // row of the chunk's first entry (the last r with Mp[r] <= base,
-        // searched by the whole warp), then each lane walks forward
+        // searched by the whole warp), then each lane's
         const int32_t r0 = warp_last_le<int32_t, int32_t>(Mp, (int32_t)nrows, (int32_t)base,
                                                           lane);
-        int32_t i = r0;
-        if (valid) while (Mp[i + 1] <= pm) i++;
+        const int32_t i = warp_rows<int32_t, int32_t>(
+            Mp, (int32_t)nrows, r0, (int32_t)(valid ? pm : mnz - 1), lane);
         int32_t j = 0, a0 = 0, a1 = 0, b0 = 0, b1 = 0;
         bool coop = false, exists = false;
         Z cij = Z();
@@ -433,8 +433,8 @@ k_ct_classify(const int32_t *__restrict__ Mp, const int32_t *__restrict__ Mj,
         const bool valid = pm < mnz;
         const int32_t r0 = warp_last_le<int32_t, int32_t>(Mp, (int32_t)nrows, (int32_t)base,
                                                           lane);
-        int32_t i = r0;
-        if (valid) while (Mp[i + 1] <= pm) i++;
+        const int32_t i = warp_rows<int32_t, int32_t>(
+            Mp, (int32_t)nrows, r0, (int32_t)(valid ? pm : mnz - 1), lane);
         int32_t key = -1, q0 = 0, q1 = 0;
         if (valid) {
             const int32_t j = Mj[pm];

@@ -163,6 +163,10 @@ int dev_mask_to_struct(DevCSR &out, const DevCSR &M, cudaStream_t s);
 // remove zombies in place (GB_wait's zombie pruning), producing a clean CSR
 int dev_prune_zombies(DevCSR &A, cudaStream_t s);
 
+// *inside = every live entry of C is an entry of M (false, without a look,
+// where C or M holds zombies)
+int dev_inside(const DevCSR &C, const DevCSR &M, bool *inside, cudaStream_t s);
+
 // upload from the caller's int64 CSR with checks on the device (offsets from
 // 0 to nnz, never decreasing; indices in [0, ncols); rows given out of order
 // are sorted, duplicates rejected): INVALID_OBJECT when the arrays are not a
@@ -180,10 +184,7 @@ int dev_download_to(const DevCSR &A, int64_t *p, int64_t *i, void *x, cudaStream
 int dev_copy_out(const DevCSR &A, int64_t *p, int64_t *i, void *x, cudaStream_t s);
 
 // ---- scans ----
-// exclusive scan of n int64 values in place; out[n] receives the total when
-// `with_total`.  `in` and `out` may alias.
-int scan_exclusive_i64(const int64_t *in, int64_t *out, int64_t n,
-                       cudaStream_t s);
+// exclusive scan of n values
 int scan_exclusive_i32_to_i64(const int32_t *in, int64_t *out, int64_t n,
                               cudaStream_t s);
 // allocation-free variant: ws holds scan_ws_elems(n) int64 values

@@ -1,0 +1,85 @@
+"""C<M> = T without replace (GrB_mxm under a plain structural mask): a C that
+lies inside M becomes T, any other is merged with it; and the zombie pruning
+behind it, at the edges of its tiles.  Checked against the oracle."""
+
+import numpy as np
+import pytest
+
+from graphblas_b200 import workloads as W
+from tests.helpers import assert_exact, random_csr
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def api(gpu):
+    from graphblas_b200.grb import API
+    return API()
+
+
+def subset(M, keep, dtype):
+    """The entries of M where keep, with values of their own."""
+    rows = np.repeat(np.arange(M.nrows), np.diff(M.p))[keep]
+    p = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=M.nrows))]).astype(np.int64)
+    i = M.i[keep]
+    return W.Csr(M.nrows, M.ncols, p, i, (100 + np.arange(len(i))).astype(dtype))
+
+
+def with_outside(C, M):
+    """C with one entry added that M does not hold (in the first row with room)."""
+    for r in range(M.nrows):
+        free = np.setdiff1d(np.arange(M.ncols), M.i[M.p[r]:M.p[r + 1]])
+        if len(free):
+            j = free[-1]
+            at = C.p[r] + np.searchsorted(C.i[C.p[r]:C.p[r + 1]], j)
+            p = C.p.copy()
+            p[r + 1:] += 1
+            return W.Csr(C.nrows, C.ncols, p, np.insert(C.i, at, j), np.insert(C.x, at, 7))
+    raise AssertionError("M is full")
+
+
+# (rows, columns, density of M): a few entries; one entry short of, at and past
+# a tile of 2048; several tiles with empty rows and zombies in every chunk
+SHAPES = [(3, 40, 0.2), (23, 89, 1.0), (32, 64, 1.0), (3, 683, 1.0), (400, 300, 0.12)]
+
+
+@pytest.mark.parametrize("m,n,density", SHAPES)
+@pytest.mark.parametrize("name,tc,np_t", [("GrB_PLUS_TIMES_SEMIRING_FP64", 11, np.float64),
+                                          ("GrB_MIN_PLUS_SEMIRING_FP32", 10, np.float32),
+                                          ("GxB_PLUS_PAIR_INT64", 8, np.int64),
+                                          ("GrB_LOR_LAND_SEMIRING_BOOL", 1, np.bool_)])
+@pytest.mark.parametrize("start", ["inside", "outside", "same", "more"])
+def test_masked_write_without_replace(api, oracle, m, n, density, name, tc, np_t, start):
+    k = 60
+    A, B = random_csr(m, k, 0.06, 1, np_t), random_csr(n, k, 0.06, 2, np_t)
+    M = random_csr(m, n, density, 3, np_t)
+    add, mult = {11: ("PLUS", "TIMES"), 10: ("MIN", "PLUS"), 8: ("PLUS", "PAIR"),
+                 1: ("LOR", "LAND")}[tc]
+    T = oracle.dot3(m, n, (A.p, A.i, A.x, tc), (B.p, B.i, B.x, tc), (M.p, M.i, None, 1), add,
+                    mult, tc)
+    if start == "same":
+        C = W.Csr(m, n, T[0], T[1], T[2].copy())
+    else:
+        C = subset(M, np.arange(M.nnz) % 3 != 1, np_t)
+    if start in ("outside", "more"):
+        if density == 1.0:
+            pytest.skip("every column is in M")
+        C = with_outside(C, M)
+    if start == "more":                     # more entries than M has
+        full = random_csr(m, n, 1.0, 5, np_t)
+        C = subset(full, np.ones(full.nnz, bool), np_t)
+    want = oracle.accum_mask(m, n, (C.p, C.i, C.x), T, tc, M=(M.p, M.i, None, 1),
+                             mask_struct=True, mask_comp=False, replace=False, accum=None)
+    hA, hB, hM = (api.matrix_from_csr(X, tc) for X in (A, B, M))
+    hC = api.matrix_from_csr(C, tc)
+    for _ in range(2):                      # the second call finds the first one's result
+        api.mxm(hC, hM, None, name, hA, hB, "GrB_DESC_ST1")
+        assert api.nvals(hC) == len(want[1])
+    if tc == 8:
+        assert api.reduce(hC, "GrB_PLUS_MONOID_INT64", 8) == int(np.sum(want[2]))
+    # the result is a mask like any other: it holds no zombies
+    hD = api.matrix_new(tc, m, n)
+    api.mxm(hD, hC, None, name, hA, hB, "GrB_DESC_ST1")
+    assert_exact(api.matrix_to_csr(hC, tc, m), want, "C<M> = T")
+    for X in (hA, hB, hM, hC, hD):
+        api.free(X)
