@@ -109,11 +109,12 @@ k_flops_flat(const int32_t *__restrict__ Ap, const int32_t *__restrict__ Aj,
         unsigned long long carry = 0;
         for (int64_t base = s0; base < s1; base += 32) {
             const int64_t e = base + lane;
-            int32_t r = -1;
+            int32_t r = warp_rows<int32_t, int32_t>(Ap, (int32_t)nrows, r0,
+                                                    (int32_t)(e < s1 ? e : s1 - 1), lane);
             unsigned long long f = 0;
-            if (e < s1) {
-                r = r0;
-                while (Ap[r + 1] <= e) r++;
+            if (e >= s1) {
+                r = -1;
+            } else {
                 const int32_t k = Aj[e];
                 f = (unsigned long long)(Bp[k + 1] - Bp[k]);
             }
@@ -406,95 +407,193 @@ k_saxpy_hash(BinRows br, int tpr_log2, int cap,
 // so every semiring, floating PLUS included, gives the same bits.
 static constexpr int ESC_WARPS = 8;
 
-// Bitonic sort of a warp's n <= 32*R keys in registers: element e = 32*r +
-// lane sits in k[r]; compare-exchanges with strides of 32 or more stay inside
-// a lane, shorter ones go through shuffles.  Keys past n sort as all ones.
-// The keys are read from and written back to key[0..n).
+// Sort of a warp's 32*R keys held in registers, key e = lane*R + r of the
+// sorted order in k[r] of its lane.  A bitonic network with every exchange
+// ascending (a merge starts by comparing e with its mirror image in the pair
+// of runs), so an exchange is one min and one max, or one of the two across
+// lanes.  With consecutive keys in a lane the strides below R stay in
+// registers: 64 + 40 exchanges of a 256-key sort are 15 shuffle steps, where
+// keys 32 apart in a lane took 30.
 template <int R, typename KT>
-__device__ __forceinline__ void warp_sort_regs(KT *key, int n, int lane)
+__device__ __forceinline__ void warp_sort_blocked(KT (&k)[R], int lane)
 {
-    KT k[R];
-    #pragma unroll
-    for (int r = 0; r < R; r++) {
-        const int e = r * 32 + lane;
-        k[r] = e < n ? key[e] : ~(KT)0;
-    }
     #pragma unroll
     for (int size = 2; size <= 32 * R; size <<= 1) {
+        if (size <= R) {
+            #pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int q = r ^ (size - 1);
+                if (q > r) {
+                    const KT a = k[r], b = k[q];
+                    k[r] = min(a, b);
+                    k[q] = max(a, b);
+                }
+            }
+        } else {
+            const int lm = size / R - 1;
+            const bool lower = (lane & (size / (2 * R))) == 0;
+            KT o[R];
+            #pragma unroll
+            for (int r = 0; r < R; r++) o[r] = __shfl_xor_sync(0xffffffffu, k[R - 1 - r], lm);
+            #pragma unroll
+            for (int r = 0; r < R; r++) k[r] = lower ? min(k[r], o[r]) : max(k[r], o[r]);
+        }
         #pragma unroll
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            if (stride >= 32) {
-                const int rs = stride >> 5;
+        for (int stride = size >> 2; stride > 0; stride >>= 1) {
+            if (stride < R) {
                 #pragma unroll
                 for (int r = 0; r < R; r++) {
-                    if (r & rs) continue;
-                    const int r2 = r | rs;
-                    const bool up = ((r * 32 + lane) & size) == 0;
-                    const KT a = k[r], b = k[r2];
-                    const KT lo = a < b ? a : b, hi = a < b ? b : a;
-                    k[r] = up ? lo : hi;
-                    k[r2] = up ? hi : lo;
+                    if (r & stride) continue;
+                    const KT a = k[r], b = k[r | stride];
+                    k[r] = min(a, b);
+                    k[r | stride] = max(a, b);
                 }
             } else {
+                const int lm = stride / R;
+                const bool lower = (lane & lm) == 0;
                 #pragma unroll
                 for (int r = 0; r < R; r++) {
-                    const KT other = __shfl_xor_sync(0xffffffffu, k[r], stride);
-                    const bool up = ((r * 32 + lane) & size) == 0;
-                    const bool lower = (lane & stride) == 0;
-                    k[r] = (lower == up) ? (k[r] < other ? k[r] : other)
-                                         : (k[r] < other ? other : k[r]);
+                    const KT o = __shfl_xor_sync(0xffffffffu, k[r], lm);
+                    k[r] = lower ? min(k[r], o) : max(k[r], o);
                 }
             }
         }
     }
+}
+
+// an entry A(i,k) of the row being expanded: position of B(k,0) less the
+// products before it (so that product q is B's entry base + q), k and A(i,k)
+template <typename Z> struct __align__(16) EscEnt { int32_t base, k; Z a; };
+static constexpr int ESC_ENTS = 32;              // entries of A a warp stages at a time
+
+// The operands of a row's expansion
+struct EscIn {
+    const int32_t *Ap, *Aj;
+    const void *Ax;
+    const int32_t *Bp, *Bj;
+    const void *Bx;
+    const int32_t *Mp, *Mj;
+    bool a_iso, b_iso, has_mask, mask_comp;
+};
+
+__device__ __forceinline__ bool esc_allowed(const EscIn &in, int32_t m0, int32_t m1, int32_t j)
+{
+    const int32_t f = lower_bound(in.Mj, m0, m1, j);
+    const bool present = f < m1 && in.Mj[f] == j;
+    return in.mask_comp ? !present : present;
+}
+
+// A row of at most 32*R products whose entries of A are staged in ent[]:
+// lane's entry (if it has products) starts at product `excl`.  A product's
+// entry is the number of starts at or before it: the starts that fall in 32
+// consecutive products come as one word (one reduction), so no product
+// searches.  All of the row's columns and values are in flight at once.
+// Products outside the mask sort to the end.  On return kp[0..n) are the
+// sorted keys (column << posb | product), vp[] the products' values by
+// product; heads = the row's distinct columns.
+template <class SR, typename KT, int R>
+__device__ __forceinline__ void esc_fast(int32_t i, int total, int excl, bool has, int posb,
+                                         KT *kp, typename SR::z_t *vp,
+                                         const EscEnt<typename SR::z_t> *ent, const EscIn &in,
+                                         int &n, int &heads)
+{
+    using Z = typename SR::z_t;
+    const int lane = threadIdx.x & 31;
+    const unsigned upto = 0xffffffffu >> (31 - lane);
+    constexpr int G = R < 4 ? R : 4;
+    int32_t m0 = 0, m1 = 0;
+    if (in.has_mask) { m0 = in.Mp[i]; m1 = in.Mp[i + 1]; }
+    KT key[R];
+    int c = -1, kept = 0;
+    #pragma unroll
+    for (int g = 0; g < R; g += G) {
+        int32_t j[G];
+        int src[G];
+        Z b[G];
+        #pragma unroll
+        for (int u = 0; u < G; u++) {
+            const unsigned st = __reduce_or_sync(
+                0xffffffffu, has && (excl >> 5) == g + u ? 1u << (excl & 31) : 0u);
+            src[u] = c + __popc(st & upto);
+            c += __popc(st);
+            const int q = (g + u) * 32 + lane;
+            j[u] = -1;
+            b[u] = Z();
+            if (q < total) {
+                const int32_t pb = ent[src[u]].base + q;
+                j[u] = in.Bj[pb];
+                if (SR::needs_b) b[u] = ld_val<Z>(in.Bx, pb, in.b_iso);
+            }
+        }
+        #pragma unroll
+        for (int u = 0; u < G; u++) {
+            const int q = (g + u) * 32 + lane;
+            bool keep = j[u] >= 0;
+            if (in.has_mask) {
+                if (keep) keep = esc_allowed(in, m0, m1, j[u]);
+                kept += __popc(__ballot_sync(0xffffffffu, keep));
+            }
+            key[g + u] = ~(KT)0;
+            if (keep) {
+                const EscEnt<Z> e = ent[src[u]];
+                key[g + u] = ((KT)(uint32_t)j[u] << posb) | (KT)q;
+                vp[q] = SR::F::f(e.a, b[u], i, e.k, j[u]);
+            }
+        }
+    }
+    n = in.has_mask ? kept : total;
+    warp_sort_blocked<R, KT>(key, lane);
+    const KT before = __shfl_up_sync(0xffffffffu, key[R - 1], 1);
+    int h = 0;
     #pragma unroll
     for (int r = 0; r < R; r++) {
-        const int e = r * 32 + lane;
-        if (e < n) key[e] = k[r];
+        const KT p = r ? key[r - 1] : before;
+        h += lane * R + r < n && (lane * R + r == 0 || (p >> posb) != (key[r] >> posb));
+    }
+    heads = __reduce_add_sync(0xffffffffu, h);
+    // whole vectors: the keys after n inside the last one are never read
+    // (kp is 16-byte aligned with room for a multiple of 8 keys)
+    if constexpr (sizeof(KT) == 4 && R >= 4) {
+        #pragma unroll
+        for (int r = 0; r < R; r += 4)
+            if (lane * R + r < n)
+                *reinterpret_cast<uint4 *>(kp + lane * R + r) =
+                    make_uint4(key[r], key[r + 1], key[r + 2], key[r + 3]);
+    } else {
+        #pragma unroll
+        for (int r = 0; r < R; r++)
+            if (lane * R + r < n) kp[lane * R + r] = key[r];
     }
 }
 
-// One row of the expand-sort-compress bin by one warp: the row's products
-// (at most cap) expand into key[] / val[] (the warp's shared-memory arrays),
-// the keys are sorted and each run of equal columns is folded into one entry
-// of Tj / Tx from position off() on (read only when the row is written).
-// Returns the row's entry count; with LIMIT, -1 (and nothing written) when
-// the row keeps more than cap products.
-// KT: 32-bit keys when (column << posb) fits, else 64-bit; posb = log2(cap)
-// bits hold the product's position, so only the keys move in the sort and
-// the values stay where the expansion wrote them.
-template <class SR, typename KT, bool LIMIT = false, class Off>
-__device__ __forceinline__ int esc_row(int32_t i, int cap, int posb, KT *key,
-                                       typename SR::z_t *val,
-                                       const int32_t *__restrict__ Ap,
-                                       const int32_t *__restrict__ Aj,
-                                       const void *__restrict__ Ax, bool a_iso,
-                                       const int32_t *__restrict__ Bp,
-                                       const int32_t *__restrict__ Bj,
-                                       const void *__restrict__ Bx, bool b_iso,
-                                       const int32_t *__restrict__ Mp,
-                                       const int32_t *__restrict__ Mj,
-                                       bool has_mask, bool mask_comp, const Off &off_of,
-                                       int32_t *__restrict__ Tj, typename SR::z_t *__restrict__ Tx)
+// Row i's products expanded and sorted by one warp into kp / vp (cap
+// entries): see esc_fast.  Rows past 32 entries of A, or past 256 products
+// before the mask, take the loop below, which keeps only the products inside
+// the mask.  Returns n, the products kept, or -1 when there are more than
+// cap of them; span = the places of vp that they lie in.
+template <class SR, typename KT>
+__device__ __forceinline__ int esc_sort_row(int32_t i, int cap, int posb, KT *kp,
+                                            typename SR::z_t *vp,
+                                            EscEnt<typename SR::z_t> *ent, const EscIn &in,
+                                            int &heads, int &span)
 {
     using Z = typename SR::z_t;
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
-    const KT posmask = ((KT)1 << posb) - 1;
-    const int32_t pa0 = Ap[i], pa1 = Ap[i + 1];
-    int32_t m0 = 0, m1 = 0;
-    if (has_mask) { m0 = Mp[i]; m1 = Mp[i + 1]; }
-    int n = 0;                                   // products kept so far
-    for (int32_t c0 = pa0; c0 < pa1; c0 += 32) {
+    const int32_t pa0 = in.Ap[i], pa1 = in.Ap[i + 1];
+    heads = 0;
+    span = 0;
+    int n = 0;
+    for (int32_t c0 = pa0; c0 < pa1; c0 += ESC_ENTS) {
         // 32 entries of A(i,:) at a time: lane l holds k and nnz(B(k,:))
         const int32_t pa = c0 + lane;
         int32_t k = 0, b0 = 0, len = 0;
         Z a = Z();
         if (pa < pa1) {
-            k = Aj[pa];
-            b0 = Bp[k];
-            len = Bp[k + 1] - b0;
-            if (SR::needs_a) a = ld_val<Z>(Ax, pa, a_iso);
+            k = in.Aj[pa];
+            b0 = in.Bp[k];
+            len = in.Bp[k + 1] - b0;
+            if (SR::needs_a) a = ld_val<Z>(in.Ax, pa, in.a_iso);
         }
         int incl = len;
         #pragma unroll
@@ -503,178 +602,206 @@ __device__ __forceinline__ int esc_row(int32_t i, int cap, int posb, KT *key,
             if (lane >= o) incl += y;
         }
         const int total = __shfl_sync(0xffffffffu, incl, 31);
+        const int excl = incl - len;
+        const unsigned vm = __ballot_sync(0xffffffffu, len > 0);
+        __syncwarp();                            // the last chunk's entries are read
+        if (len > 0) ent[__popc(vm & below)] = EscEnt<Z>{b0 - excl, k, a};
+        __syncwarp();
+        if (pa1 - pa0 <= ESC_ENTS && total <= 256 && total <= cap) {
+            if (total == 0) return 0;
+            span = total;
+            if (total <= 32) esc_fast<SR, KT, 1>(i, total, excl, len > 0, posb, kp, vp, ent, in, n, heads);
+            else if (total <= 64) esc_fast<SR, KT, 2>(i, total, excl, len > 0, posb, kp, vp, ent, in, n, heads);
+            else if (total <= 128) esc_fast<SR, KT, 4>(i, total, excl, len > 0, posb, kp, vp, ent, in, n, heads);
+            else esc_fast<SR, KT, 8>(i, total, excl, len > 0, posb, kp, vp, ent, in, n, heads);
+            __syncwarp();
+            return n;
+        }
+        int c = -1;
+        int32_t m0 = 0, m1 = 0;
+        if (in.has_mask) { m0 = in.Mp[i]; m1 = in.Mp[i + 1]; }
         for (int q0 = 0; q0 < total; q0 += 32) {
-            // product q of this chunk belongs to the first lane src whose
-            // inclusive count exceeds q
+            const unsigned st = __reduce_or_sync(
+                0xffffffffu, len > 0 && (excl >> 5) == (q0 >> 5) ? 1u << (excl & 31) : 0u);
+            const int src = c + __popc(st & (below | (1u << lane)));
+            c += __popc(st);
             const int q = q0 + lane;
-            int src = 0;
-            #pragma unroll
-            for (int step = 16; step > 0; step >>= 1) {
-                const int v = __shfl_sync(0xffffffffu, incl, src + step - 1);
-                if (v <= q) src += step;
-            }
-            const int excl = __shfl_sync(0xffffffffu, incl - len, src);
-            const int32_t kk = __shfl_sync(0xffffffffu, k, src);
-            const int32_t bb = __shfl_sync(0xffffffffu, b0, src);
-            const Z aa = shfl<Z>(a, src);
             bool keep = q < total;
             int32_t j = 0, pb = 0;
             if (keep) {
-                pb = bb + (q - excl);
-                j = Bj[pb];
-                if (has_mask) {
-                    const int32_t f = lower_bound(Mj, m0, m1, j);
-                    const bool present = f < m1 && Mj[f] == j;
-                    keep = mask_comp ? !present : present;
-                }
+                pb = ent[src].base + q;
+                j = in.Bj[pb];
+                if (in.has_mask) keep = esc_allowed(in, m0, m1, j);
             }
             const unsigned km = __ballot_sync(0xffffffffu, keep);
-            if (LIMIT && n + __popc(km) > cap) return -1;
+            if (n + __popc(km) > cap) return -1;
             if (keep) {
                 const int pos = n + __popc(km & below);
+                const EscEnt<Z> e = ent[src];
                 Z b = Z();
-                if (SR::needs_b) b = ld_val<Z>(Bx, pb, b_iso);
-                key[pos] = ((KT)(uint32_t)j << posb) | (KT)pos;
-                val[pos] = SR::F::f(aa, b, i, kk, j);
+                if (SR::needs_b) b = ld_val<Z>(in.Bx, pb, in.b_iso);
+                kp[pos] = ((KT)(uint32_t)j << posb) | (KT)pos;
+                vp[pos] = SR::F::f(e.a, b, i, e.k, j);
             }
             n += __popc(km);
         }
     }
     __syncwarp();
-    int n2 = 1;
-    while (n2 < n) n2 <<= 1;
-    if (n <= 32) {
-        // one key per lane: bitonic network over the lanes in registers
-        KT kk = lane < n ? key[lane] : ~(KT)0;
+    // the keys sorted: up to 256 in registers, more by a bitonic network in
+    // shared memory (a lane owns every 32nd compare-exchange)
+    if (n <= 256) {
+        KT key[8];
         #pragma unroll
-        for (int size = 2; size <= 32; size <<= 1) {
-            #pragma unroll
+        for (int r = 0; r < 8; r++) key[r] = r * 32 + lane < n ? kp[r * 32 + lane] : ~(KT)0;
+        __syncwarp();
+        warp_sort_blocked<8, KT>(key, lane);
+        #pragma unroll
+        for (int r = 0; r < 8; r++)
+            if (lane * 8 + r < n) kp[lane * 8 + r] = key[r];
+    } else {
+        int n2 = 1;
+        while (n2 < n) n2 <<= 1;
+        for (int q = n + lane; q < n2; q += 32) kp[q] = ~(KT)0;
+        __syncwarp();
+        for (int size = 2; size <= n2; size <<= 1) {
             for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                const KT other = __shfl_xor_sync(0xffffffffu, kk, stride);
-                const bool up = (lane & size) == 0;
-                const bool lower = (lane & stride) == 0;
-                kk = (lower == up) ? (kk < other ? kk : other) : (kk < other ? other : kk);
+                for (int q = lane; q < (n2 >> 1); q += 32) {
+                    // q-th pair of this pass: lower index a, partner a + stride
+                    const int a = ((q & ~(stride - 1)) << 1) | (q & (stride - 1));
+                    const int b = a + stride;
+                    const bool up = ((a & size) == 0);
+                    const KT ka = kp[a], kb = kp[b];
+                    if ((ka > kb) == up) { kp[a] = kb; kp[b] = ka; }
+                }
+                __syncwarp();
             }
         }
-        if (lane < n) key[lane] = kk;
-        n2 = 0;                                  // the shared-memory network is skipped
-    } else if (n <= 64) {
-        warp_sort_regs<2>(key, n, lane);
-        n2 = 0;
-    } else if (n <= 128) {
-        warp_sort_regs<4>(key, n, lane);
-        n2 = 0;
-    } else if (n <= 256) {
-        warp_sort_regs<8>(key, n, lane);
-        n2 = 0;
     }
-    for (int q = n + lane; q < n2; q += 32) key[q] = ~(KT)0;
     __syncwarp();
-    // bitonic sort of the keys; a lane owns every 32nd compare-exchange
-    for (int size = 2; size <= n2; size <<= 1) {
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int q = lane; q < (n2 >> 1); q += 32) {
-                // q-th pair of this pass: lower index a, partner a + stride
-                const int a = ((q & ~(stride - 1)) << 1) | (q & (stride - 1));
-                const int b = a + stride;
-                const bool up = ((a & size) == 0);
-                const KT ka = key[a], kb = key[b];
-                if ((ka > kb) == up) { key[a] = kb; key[b] = ka; }
-            }
-            __syncwarp();
+    int h = 0;
+    for (int p = lane; p < n; p += 32) h += p == 0 || (kp[p - 1] >> posb) != (kp[p] >> posb);
+    heads = __reduce_add_sync(0xffffffffu, h);
+    span = n;
+    return n;
+}
+
+// The sorted products of a row folded into its entries, written from Tj / Tx
+// on: the first product of each run of equal columns folds the run in
+// ascending k (its positions ascend).
+template <class SR, typename KT>
+__device__ __forceinline__ void esc_fold(int n, int heads, int posb, const KT *kp,
+                                         const typename SR::z_t *vp, int32_t *__restrict__ Tj,
+                                         typename SR::z_t *__restrict__ Tx)
+{
+    using Z = typename SR::z_t;
+    const int lane = threadIdx.x & 31;
+    const KT posmask = ((KT)1 << posb) - 1;
+    if (heads == n) {                            // no two products meet
+        for (int p = lane; p < n; p += 32) {
+            const KT k = kp[p];
+            Tj[p] = (int32_t)(k >> posb);
+            Tx[p] = vp[k & posmask];
         }
+        return;
     }
-    // the first entry of each run of equal columns folds the run in
-    // ascending k (its positions ascend) and writes one output entry
-    const int64_t off = off_of();
+    const unsigned below = (1u << lane) - 1u;
     int out = 0;
     for (int c0 = 0; c0 < n; c0 += 32) {
         const int p = c0 + lane;
         bool head = false;
-        KT kp = 0;
+        KT k = 0;
         if (p < n) {
-            kp = key[p];
-            head = (p == 0) || ((key[p - 1] >> posb) != (kp >> posb));
+            k = kp[p];
+            head = p == 0 || (kp[p - 1] >> posb) != (k >> posb);
         }
         const unsigned hm = __ballot_sync(0xffffffffu, head);
         if (head) {
-            const KT jcol = kp >> posb;
-            Z z = val[kp & posmask];
+            const KT jcol = k >> posb;
+            Z z = vp[k & posmask];
             for (int r = p + 1; r < n; r++) {
-                const KT kr = key[r];
+                const KT kr = kp[r];
                 if ((kr >> posb) != jcol) break;
-                z = SR::M::update(z, val[kr & posmask]);
+                z = SR::M::update(z, vp[kr & posmask]);
             }
-            const int64_t dst = off + out + __popc(hm & below);
+            const int dst = out + __popc(hm & below);
             Tj[dst] = (int32_t)jcol;
             Tx[dst] = z;
         }
         out += __popc(hm);
     }
-    return out;
 }
 
 template <class SR, typename KT>
-__global__ void __launch_bounds__(ESC_WARPS * 32, 6)
-k_saxpy_esc(BinRows br, int cap, int posb,
-            const int32_t *__restrict__ Ap, const int32_t *__restrict__ Aj,
-            const void *__restrict__ Ax, bool a_iso,
-            const int32_t *__restrict__ Bp, const int32_t *__restrict__ Bj,
-            const void *__restrict__ Bx, bool b_iso,
-            const int32_t *__restrict__ Mp, const int32_t *__restrict__ Mj,
-            bool has_mask, bool mask_comp,
-            const int64_t *__restrict__ slot_off,
+__global__ void __launch_bounds__(ESC_WARPS * 32, 4)
+k_saxpy_esc(BinRows br, int cap, int posb, EscIn in, const int64_t *__restrict__ slot_off,
             int32_t *__restrict__ Tj, typename SR::z_t *__restrict__ Tx,
             int32_t *__restrict__ row_cnt)
 {
     using Z = typename SR::z_t;
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ EscEnt<Z> s_ent[ESC_WARPS][ESC_ENTS];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    KT *key = (KT *)(smem + (size_t)w * cap * (sizeof(KT) + sizeof(Z)));
-    Z *val = (Z *)((unsigned char *)key + (size_t)cap * sizeof(KT));
+    Z *vp = (Z *)(smem + (size_t)w * cap * (sizeof(KT) + sizeof(Z)));
+    KT *kp = (KT *)((unsigned char *)vp + (size_t)cap * sizeof(Z));
     const int32_t *rows;
     const int nrows_bin = br.get(rows);
 
     for (int64_t rb = (int64_t)blockIdx.x * ESC_WARPS + w; rb < nrows_bin;
          rb += (int64_t)gridDim.x * ESC_WARPS) {
         const int32_t i = rows[rb];
-        const int out = esc_row<SR, KT>(i, cap, posb, key, val, Ap, Aj, Ax, a_iso, Bp, Bj, Bx,
-                                        b_iso,
-                                        Mp, Mj, has_mask, mask_comp,
-                                        [&]() { return slot_off[i]; }, Tj, Tx);
-        if (lane == 0) row_cnt[i] = out;
+        int heads, span;
+        const int n = esc_sort_row<SR, KT>(i, cap, posb, kp, vp, s_ent[w], in, heads, span);
+        const int64_t off = slot_off[i];
+        esc_fold<SR, KT>(n, heads, posb, kp, vp, Tj + off, Tx + off);
+        if (lane == 0) row_cnt[i] = heads;
         __syncwarp();
     }
 }
 
 // ---------------------------------------------------------------------------
-// small products in one launch
+// products of short rows in one launch
 // ---------------------------------------------------------------------------
 
 // C = A*B (masked or not) in one launch, for products whose rows all fit the
-// expand-sort-compress bin.  Blocks take row ranges of `chunk` rows from a
-// ticket in the order they start, and row i's slots are [i*SMALL_CAP,
-// (i+1)*SMALL_CAP):
+// expand-sort-compress bin (at most SMALL_CAP products kept).  Blocks take
+// ranges of `chunk` rows from a ticket in the order they start:
 //
-//   1. each row expands, sorts and compresses into its slots (esc_row); a
-//      row that keeps more than SMALL_CAP products sets tot[1] instead
+//   1. each row expands and sorts into its warp's arena in shared memory and
+//      stays there; only its entry count is known now.  A warp whose arena
+//      is full folds its rows into the spill buffer (space from a cursor)
+//      and starts over; rows past SMALL_CAP products set tot[1].
 //   2. the block's entry count is posted, and a decoupled look-back over the
 //      blocks before it (they started earlier, so they are running or done)
 //      gives its offset among C's entries; the last block's inclusive sum is
 //      nnz(C)
-//   3. C's row offsets for the block's rows, and its entries copied from the
-//      slots, flat over the block's threads
+//   3. each warp folds its rows from the arena straight into C, and the
+//      block writes its rows' offsets.
+//
+// Bound by instruction issue and by L2 latency (the gathers of B's rows), so
+// every entry crosses memory once: no slots, and no pass that packs them.
+// 65536 rows of 4-16 entries (6.5M products, fp64): 142 us, where the
+// separate flop count, bins, slots, row offsets and pack took 200 us.
+// A 24 KB arena of 512 12-byte products a warp holds four rows of a hundred
+// products, so that a block's look-back is paid once for 32 rows.
 //
 // No block waits for one that has not started, so the launch needs no
-// co-residency and runs beside other kernels.  tot[0] = nnz(C), tot[1] = 0
-// (done), SMALL_TOO_LONG or SMALL_NO_ROOM (C's arrays too small; the blocks
-// past the capacity write nothing), tot[2] is set when a look-back gave up
-// waiting (the results are void), tot[3] is the ticket counter; part[G] are
-// the blocks' look-back words.  The host zeroes tot[] and part[] first.
+// co-residency and runs beside other kernels.  tot[1] = 0 (done),
+// SMALL_TOO_LONG or SMALL_NO_ROOM (C's arrays or the spill buffer too small;
+// the blocks past the capacity write nothing), tot[2] is set when a look-back
+// gave up waiting (the results are void), tot[3] is the ticket counter,
+// tot[4] the spill cursor; part[G] are the blocks' look-back words.  The host
+// zeroes tot[] and part[] first; tot[0] = nnz(C).
 static constexpr int SMALL_CAP = 256;              // products per row, at most
 static constexpr int SMALL_POSB = 8;               // log2(SMALL_CAP)
 static constexpr int SMALL_CHUNK = 128;            // rows per block, at most
+static constexpr int SMALL_ARENA = 6144;           // bytes of products a warp holds
+static constexpr int64_t SMALL_MIN_ROWS = 2;       // rows of a product, at least
 enum { SMALL_DONE = 0, SMALL_TOO_LONG = 1, SMALL_NO_ROOM = 3 };
+
+template <typename Z> __host__ __device__ constexpr int small_arena_entries()
+{
+    return SMALL_ARENA / (int)(4 + sizeof(Z)) / 16 * 16;
+}
 
 // exclusive scan of v[0..n) (n <= SMALL_CHUNK) in place by warp 0; returns
 // the total to every lane of warp 0
@@ -708,57 +835,95 @@ __device__ __forceinline__ T small_warp_scan(T *v, int n, int lane)
 }
 
 template <class SR>
-__global__ void __launch_bounds__(ESC_WARPS * 32, 6)
-k_saxpy_small(int32_t m, int32_t chunk,
-              const int32_t *__restrict__ Ap, const int32_t *__restrict__ Aj,
-              const void *__restrict__ Ax, bool a_iso,
-              const int32_t *__restrict__ Bp, const int32_t *__restrict__ Bj,
-              const void *__restrict__ Bx, bool b_iso,
-              const int32_t *__restrict__ Mp, const int32_t *__restrict__ Mj,
-              bool has_mask, bool mask_comp, long long *__restrict__ part,
-              int32_t *__restrict__ Tj, typename SR::z_t *__restrict__ Tx,
+__global__ void __launch_bounds__(ESC_WARPS * 32, 4)
+k_saxpy_small(int32_t m, int32_t chunk, EscIn in, long long *__restrict__ part,
+              int32_t *__restrict__ Sj, typename SR::z_t *__restrict__ Sx, int64_t scap,
               int32_t *__restrict__ Cp, int32_t *__restrict__ Cj,
               typename SR::z_t *__restrict__ Cx, int64_t ccap, long long *__restrict__ tot)
 {
     using Z = typename SR::z_t;
     using KT = uint32_t;
+    constexpr int ACAP = small_arena_entries<Z>();
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ EscEnt<Z> s_ent[ESC_WARPS][ESC_ENTS];
     __shared__ int s_cnt[SMALL_CHUNK];           // the rows' entry counts
+    __shared__ int s_n[SMALL_CHUNK];             // their products kept
+    __shared__ int s_src[SMALL_CHUNK];           // their place in the arena, or ~place spilled
     __shared__ int s_coff[SMALL_CHUNK];          // their offsets among the block's entries
     __shared__ long long s_ex;
     __shared__ int s_btot, s_long, s_tile;
     unsigned long long *status = (unsigned long long *)part;
+    unsigned long long *utot = (unsigned long long *)tot;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int G = (int)gridDim.x;
-    // blocks take their row ranges from a ticket, in the order they start,
-    // so a block's predecessors are running or done when it looks back
+    Z *av = (Z *)(smem + (size_t)w * ACAP * (4 + sizeof(Z)));
+    KT *ak = (KT *)((unsigned char *)av + (size_t)ACAP * sizeof(Z));
     if (tid == 0) {
         s_long = 0;
-        s_tile = (int)atomicAdd((unsigned long long *)tot + 3, 1ull);
+        s_tile = (int)atomicAdd(utot + 3, 1ull);
+        // once a row was too long, the blocks that follow only pass the sum on
+        s_btot = *(volatile long long *)(tot + 1) != SMALL_DONE;
     }
     __syncthreads();
     const int b = s_tile;
     const int32_t r0 = b * chunk;
     const int32_t r1 = r0 + chunk < m ? r0 + chunk : m;
-    const int nr = r1 > r0 ? r1 - r0 : 0;
+    const int nr = r1 > r0 && !s_btot ? r1 - r0 : 0;
+    __syncthreads();
 
-    // 1. expand-sort-compress each row into its slots
-    {
-        KT *key = (KT *)(smem + (size_t)w * SMALL_CAP * (sizeof(KT) + sizeof(Z)));
-        Z *val = (Z *)((unsigned char *)key + (size_t)SMALL_CAP * sizeof(KT));
-        for (int r = w; r < nr; r += ESC_WARPS) {
-            const int32_t i = r0 + r;
-            const int out = esc_row<SR, KT, true>(i, SMALL_CAP, SMALL_POSB, key, val, Ap, Aj, Ax,
-                                                  a_iso, Bp, Bj, Bx, b_iso, Mp, Mj, has_mask,
-                                                  mask_comp,
-                                                  [&]() { return (int64_t)i * SMALL_CAP; },
-                                                  Tj, Tx);
-            if (lane == 0) {
-                s_cnt[r] = out < 0 ? 0 : out;
-                if (out < 0) s_long = 1;
+    // 1. the warp's rows into its arena
+    int used = 0, first = w;                     // the first row still in the arena
+    for (int r = w; r < nr; r += ESC_WARPS) {
+        const int32_t i = r0 + r;
+        if (used + SMALL_CAP > ACAP) {
+            // the row may not fit: its products, unless they are known to be
+            // fewer than a full row's
+            int f = 0;
+            const int32_t pa0 = in.Ap[i], pa1 = in.Ap[i + 1];
+            for (int32_t pa = pa0 + lane; pa < pa1; pa += 32) {
+                const int32_t k = in.Aj[pa];
+                f += in.Bp[k + 1] - in.Bp[k];
             }
-            __syncwarp();
+            f = __reduce_add_sync(0xffffffffu, f);
+            if (f > SMALL_CAP) f = SMALL_CAP;
+            if (used + ((f + 7) & ~7) > ACAP) {
+                for (int t = first; t < r; t += ESC_WARPS) {
+                    const int cnt = s_cnt[t];
+                    long long at = 0;
+                    if (lane == 0) at = (long long)atomicAdd(utot + 4, (unsigned long long)cnt);
+                    at = __shfl_sync(0xffffffffu, at, 0);
+                    if (at + cnt > scap) {
+                        if (lane == 0) {
+                            atomicCAS(utot + 1, 0ull, (unsigned long long)SMALL_NO_ROOM);
+                            s_cnt[t] = 0;
+                        }
+                        at = 0;
+                    } else {
+                        esc_fold<SR, KT>(s_n[t], cnt, SMALL_POSB, ak + s_src[t], av + s_src[t],
+                                         Sj + at, Sx + at);
+                    }
+                    __syncwarp();
+                    if (lane == 0) s_src[t] = ~(int)at;
+                }
+                used = 0;
+                first = r;
+                __syncwarp();
+            }
         }
+        // at most as many products as are left in the arena: a row of more
+        // than that has been given room above
+        const int room = ACAP - used < SMALL_CAP ? ACAP - used : SMALL_CAP;
+        int heads, span;
+        const int n = esc_sort_row<SR, KT>(i, room, SMALL_POSB, ak + used, av + used, s_ent[w],
+                                           in, heads, span);
+        if (lane == 0) {
+            s_cnt[r] = n < 0 ? 0 : heads;
+            s_n[r] = n < 0 ? 0 : n;
+            s_src[r] = used;
+            if (n < 0) s_long = 1;
+        }
+        used += (span + 7) & ~7;
+        __syncwarp();
     }
     __syncthreads();
     if (w == 0) {
@@ -768,6 +933,7 @@ k_saxpy_small(int32_t m, int32_t chunk,
         // the block's offset among C's entries: decoupled look-back over the
         // blocks before it (bounded waits; a wait past the bound sets tot[2])
         long long ex = 0;
+        if (lane == 0 && s_long) atomicExch(utot + 1, (unsigned long long)SMALL_TOO_LONG);
         if (b == 0) {
             if (lane == 0) atomicExch(&status[0], LB_INC | (unsigned long long)total);
         } else {
@@ -779,12 +945,10 @@ k_saxpy_small(int32_t m, int32_t chunk,
         if (lane == 0) {
             s_ex = ex;
             s_btot = total;
-            if (s_long) atomicExch((unsigned long long *)tot + 1, (unsigned long long)SMALL_TOO_LONG);
             if (b == G - 1) {
                 tot[0] = ex + total;
                 if (ex + total > ccap)
-                    atomicCAS((unsigned long long *)tot + 1, 0ull,
-                              (unsigned long long)SMALL_NO_ROOM);
+                    atomicCAS(utot + 1, 0ull, (unsigned long long)SMALL_NO_ROOM);
             }
         }
     }
@@ -797,31 +961,15 @@ k_saxpy_small(int32_t m, int32_t chunk,
     if (nnz_end > ccap) return;
     for (int r = tid; r < nr; r += blockDim.x) Cp[r0 + r] = (int32_t)(cbefore + s_coff[r]);
     if (r1 == m && nr > 0 && tid == 0) Cp[m] = (int32_t)nnz_end;
-    // the block's entries flat over its threads, four per thread in flight
-    const int btot = s_btot;
-    for (int e0 = tid; e0 < btot; e0 += 4 * (int)blockDim.x) {
-        int32_t jv[4];
-        Z xv[4];
-        #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int e = e0 + u * (int)blockDim.x;
-            if (e < btot) {
-                int lo = 0, hi = nr - 1;        // the last row starting at or before e
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (s_coff[mid] <= e) lo = mid; else hi = mid - 1;
-                }
-                const long long src = (long long)(r0 + lo) * SMALL_CAP + (e - s_coff[lo]);
-                jv[u] = Tj[src];
-                xv[u] = Tx[src];
-            }
-        }
-        #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int e = e0 + u * (int)blockDim.x;
-            if (e < btot) {
-                Cj[cbefore + e] = jv[u];
-                Cx[cbefore + e] = xv[u];
+    for (int r = w; r < nr; r += ESC_WARPS) {
+        const long long dst = cbefore + s_coff[r];
+        const int src = s_src[r], cnt = s_cnt[r];
+        if (src >= 0) {
+            esc_fold<SR, KT>(s_n[r], cnt, SMALL_POSB, ak + src, av + src, Cj + dst, Cx + dst);
+        } else {
+            for (int p = lane; p < cnt; p += 32) {
+                Cj[dst + p] = Sj[~src + p];
+                Cx[dst + p] = Sx[~src + p];
             }
         }
     }
@@ -1421,6 +1569,8 @@ k_pack(int64_t nrows, int span, const int64_t *__restrict__ slot_off,
             const int64_t e = base + lane;
             int64_t r = r0;
             if (e < s1) {
+                // a walk: C's rows are long (36 entries a row, 60M entries:
+                // 266 us; a search of the next 32 row starts, 369 us)
                 while (Cp64[r + 1] <= e) r++;
                 const int64_t src = slot_off[r] + (e - Cp64[r]);
                 Cj[e] = Tj[src];
@@ -1558,6 +1708,60 @@ static inline int nblocks(int64_t n, int threads, int per_sm = 8)
     int64_t cap = (int64_t)runtime().num_sms * per_sm;
     if (b > cap) b = cap;
     return b < 1 ? 1 : (int)b;
+}
+
+// blocks of a kernel that can be resident on the device at once (cached per
+// kernel and shared-memory size)
+static int resident_blocks(const void *fn, int threads, size_t smem)
+{
+    struct Entry { const void *fn; size_t smem; int blocks; };
+    static std::mutex mu;
+    static std::vector<Entry> cache;
+    std::lock_guard<std::mutex> lk(mu);
+    for (const Entry &e : cache)
+        if (e.fn == fn && e.smem == smem) return e.blocks;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem) != cudaSuccess) {
+        cudaGetLastError();
+        per_sm = 1;
+    }
+    if (per_sm < 1) per_sm = 1;
+    const int blocks = per_sm * runtime().num_sms;
+    cache.push_back({fn, smem, blocks});
+    return blocks;
+}
+
+static EscIn esc_in(const DevCSR *M, bool mask_comp, const DevCSR &A, const DevCSR &B)
+{
+    return {A.p, A.j, A.x, B.p, B.j, B.x, M ? M->p : nullptr, M ? M->j : nullptr,
+            A.iso, B.iso, M != nullptr, mask_comp};
+}
+
+// The one-launch kernel's shape for m rows of about `mean` products: rows a
+// warp (as few as fill the device in one wave, else as many as its arena
+// holds with a quarter to spare), rows a block and blocks.
+struct SmallShape { int32_t chunk; int G; size_t smem; };
+
+template <class SR>
+static SmallShape small_shape(int64_t m, double mean)
+{
+    using Z = typename SR::z_t;
+    constexpr int ACAP = small_arena_entries<Z>();
+    const size_t smem = (size_t)ESC_WARPS * ACAP * (4 + sizeof(Z));
+    static const bool once = [] {
+        allow_dynamic_smem((const void *)k_saxpy_small<SR>);
+        return true;
+    }();
+    (void)once;
+    const int64_t wave = (int64_t)resident_blocks((const void *)k_saxpy_small<SR>,
+                                                  ESC_WARPS * 32, smem) * ESC_WARPS;
+    int64_t most = (int64_t)(ACAP / (1.25 * (mean > 1.0 ? mean : 1.0)));
+    const int64_t limit = SMALL_CHUNK / ESC_WARPS;
+    most = most < 1 ? 1 : most > limit ? limit : most;
+    int64_t q = (m + wave - 1) / wave;
+    q = q < 1 ? 1 : q > most ? most : q;
+    const int64_t chunk = q * ESC_WARPS;
+    return {(int32_t)chunk, (int)((m + chunk - 1) / chunk), smem};
 }
 
 // Symbolic phase, with no host round trip: flop counts, bins and slot
@@ -1722,27 +1926,6 @@ static int plan_t(SaxpyPlan *P, const DevCSR *M, bool mask_comp, const DevCSR &A
     return cuda_to_info(cudaGetLastError());
 }
 
-// blocks of a kernel that can be resident on the device at once (cached per
-// kernel and shared-memory size)
-static int resident_blocks(const void *fn, int threads, size_t smem)
-{
-    struct Entry { const void *fn; size_t smem; int blocks; };
-    static std::mutex mu;
-    static std::vector<Entry> cache;
-    std::lock_guard<std::mutex> lk(mu);
-    for (const Entry &e : cache)
-        if (e.fn == fn && e.smem == smem) return e.blocks;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem) != cudaSuccess) {
-        cudaGetLastError();
-        per_sm = 1;
-    }
-    if (per_sm < 1) per_sm = 1;
-    const int blocks = per_sm * runtime().num_sms;
-    cache.push_back({fn, smem, blocks});
-    return blocks;
-}
-
 // Launch shared-memory bin q.  rows_bound: the bin's row count when the host
 // knows it (exact = true: an empty bin launches nothing), else an upper bound
 // (the grid is then at most one resident wave, and the kernel reads the count
@@ -1783,16 +1966,12 @@ static void launch_bin(const SaxpyPlan *P, int q, const DevCSR &A, const DevCSR 
             const int blocks = clamp(want, (const void *)k_saxpy_esc<SR, uint32_t>,
                                      ESC_WARPS * 32, sm32);
             k_saxpy_esc<SR, uint32_t><<<blocks, ESC_WARPS * 32, sm32, s>>>(br, b.cap,
-                posb, A.p, A.j, A.x, A.iso, B.p, B.j, B.x, B.iso,
-                M ? M->p : nullptr, M ? M->j : nullptr, M != nullptr, P->mask_comp,
-                P->slot_off, P->Tj, (Z *)P->Tx, P->row_cnt);
+                posb, esc_in(M, P->mask_comp, A, B), P->slot_off, P->Tj, (Z *)P->Tx, P->row_cnt);
         } else {
             const int blocks = clamp(want, (const void *)k_saxpy_esc<SR, uint64_t>,
                                      ESC_WARPS * 32, smem);
             k_saxpy_esc<SR, uint64_t><<<blocks, ESC_WARPS * 32, smem, s>>>(br, b.cap,
-                posb, A.p, A.j, A.x, A.iso, B.p, B.j, B.x, B.iso,
-                M ? M->p : nullptr, M ? M->j : nullptr, M != nullptr, P->mask_comp,
-                P->slot_off, P->Tj, (Z *)P->Tx, P->row_cnt);
+                posb, esc_in(M, P->mask_comp, A, B), P->slot_off, P->Tj, (Z *)P->Tx, P->row_cnt);
         }
     } else if (b.tpr >= 256) {
         static bool attr = false;
@@ -2064,6 +2243,18 @@ static int saxpy3_row_dense(DevCSR &C, const DevCSR *M, bool mask_comp, const De
     return SUCCESS;
 }
 
+// far more room than entries: exact arrays
+static void trim_entries(DevCSR &T, size_t zsize, cudaStream_t s)
+{
+    int32_t *j = (int32_t *)dalloc((size_t)(T.nnz + 1) * 4, s);
+    void *x = dalloc((size_t)(T.nnz + 1) * zsize, s);
+    if (!j || !x) { dfree(j, s); dfree(x, s); return; }
+    cudaMemcpyAsync(j, T.j, (size_t)T.nnz * 4, cudaMemcpyDeviceToDevice, s);
+    cudaMemcpyAsync(x, T.x, (size_t)T.nnz * zsize, cudaMemcpyDeviceToDevice, s);
+    dfree(T.j, s); dfree(T.x, s);
+    T.j = j; T.x = x;
+}
+
 // One-shot C<M> = A*B with one host round trip in the common case.  The
 // symbolic phase, the shared-memory bins, the row offsets and the pack are
 // queued together: the bins write their slots into the stream's scratch
@@ -2081,8 +2272,6 @@ static int saxpy3_row_dense(DevCSR &C, const DevCSR *M, bool mask_comp, const De
 // from B's mean row length as in the general path.  NO_VALUE when the
 // product is not taken, or when the launch found a row past the bin or too
 // little room in C (the caller then runs the general path).
-static constexpr int64_t SMALL_MIN_ROWS = 256, SMALL_MAX_ROWS = 32768;
-
 
 template <class SR>
 static int saxpy3_small(DevCSR &C, const DevCSR *M, bool mask_comp, const DevCSR &A,
@@ -2090,52 +2279,50 @@ static int saxpy3_small(DevCSR &C, const DevCSR *M, bool mask_comp, const DevCSR
 {
     using Z = typename SR::z_t;
     const int64_t m = A.nrows;
-    if (m < SMALL_MIN_ROWS || m > SMALL_MAX_ROWS || A.nnz <= 0 ||
-        B.ncols >= ((int64_t)1 << 24))
-        return NO_VALUE;
+    if (m < SMALL_MIN_ROWS || A.nnz <= 0 || B.ncols >= ((int64_t)1 << 24)) return NO_VALUE;
     const double mean_b = B.nrows > 0 ? (double)B.nnz / (double)B.nrows : 0.0;
     const double flops_est = (double)A.nnz * (mean_b > 1.0 ? mean_b : 1.0);
     if (flops_est > 0.5 * SMALL_CAP * (double)m) return NO_VALUE;
-    const size_t smem = (size_t)ESC_WARPS * SMALL_CAP * (4 + sizeof(Z));
-    const int resident = resident_blocks((const void *)k_saxpy_small<SR>, ESC_WARPS * 32, smem);
-    const int64_t chunk = (m + resident - 1) / resident;
-    if (chunk > SMALL_CHUNK) return NO_VALUE;
-    const int G = (int)((m + chunk - 1) / chunk);
+    if (1.15 * flops_est + 64.0 >= (double)INT32_MAX) return NO_VALUE;
+    const SmallShape sh = small_shape<SR>(m, flops_est / (double)m);
 
-    // one block: tot[8] and the blocks' look-back words part[G], then
-    // SMALL_CAP slots per row (values, then columns)
-    const size_t hdr = ((size_t)(8 + (size_t)G) * 8 + 255) & ~(size_t)255;
-    const size_t xbytes = ((size_t)m * SMALL_CAP * sizeof(Z) + 255) & ~(size_t)255;
-    SlotSource src(s);
-    char *base = (char *)src.get(hdr + xbytes + (size_t)m * SMALL_CAP * 4);
-    if (!base) return NO_VALUE;
+    // one block: tot[8] and the blocks' look-back words part[G], then the
+    // spill buffer (values, then columns): room for a quarter of the expected
+    // products, as rows are spilled where they are longer than expected
+    const int64_t scap = (int64_t)(flops_est / 4) + 64 * SMALL_CAP;
+    const size_t hdr = ((size_t)(8 + (size_t)sh.G) * 8 + 255) & ~(size_t)255;
+    const size_t xbytes = ((size_t)scap * sizeof(Z) + 255) & ~(size_t)255;
+    DevCSR T;
+    T.nrows = m; T.ncols = B.ncols; T.type = sr.type; T.iso = false;
+    T.p = (int32_t *)dalloc((size_t)(m + 1) * 4, s);
+    if (!T.p) return OUT_OF_MEMORY;
+    // the arrays sized from the estimate may be larger than the general path's
+    CallBlock blk(s);
+    if (!blk.get(hdr + xbytes + (size_t)scap * 4)) { dev_free(T, s); return NO_VALUE; }
+    char *base = blk.base;
     long long *tot = (long long *)base;
     long long *part = tot + 8;
-    Z *Tx = (Z *)(base + hdr);
-    int32_t *Tj = (int32_t *)(base + hdr + xbytes);
+    Z *Sx = (Z *)(base + hdr);
+    int32_t *Sj = (int32_t *)(base + hdr + xbytes);
 
     double cg = 1.15 * flops_est + 64.0;
     const double cfull = (double)m * (double)B.ncols;
     if (cg > cfull + 64.0) cg = cfull + 64.0;
     const int64_t ccap = (int64_t)cg;
-    DevCSR T;
-    T.nrows = m; T.ncols = B.ncols; T.type = sr.type; T.iso = false;
-    T.p = (int32_t *)dalloc((size_t)(m + 1) * 4, s);
     T.j = (int32_t *)dalloc((size_t)(ccap + 1) * 4, s);
     T.x = dalloc((size_t)(ccap + 1) * sizeof(Z), s);
-    if (!T.p || !T.j || !T.x) { dev_free(T, s); return NO_VALUE; }
-    cudaMemsetAsync(tot, 0, (8 + (size_t)G) * sizeof(long long), s);
+    if (!T.j || !T.x) { dev_free(T, s); return NO_VALUE; }
+    cudaMemsetAsync(tot, 0, (8 + (size_t)sh.G) * sizeof(long long), s);
     const int ps = prof_begin("saxpy3_numeric", s);
-    k_saxpy_small<SR><<<G, ESC_WARPS * 32, smem, s>>>((int32_t)m, (int32_t)chunk,
-        A.p, A.j, A.x, A.iso, B.p, B.j, B.x, B.iso,
-        M ? M->p : nullptr, M ? M->j : nullptr, M != nullptr, mask_comp,
-        part, Tj, Tx, T.p, T.j, (Z *)T.x, ccap, tot);
+    k_saxpy_small<SR><<<sh.G, ESC_WARPS * 32, sh.smem, s>>>((int32_t)m, sh.chunk,
+        esc_in(M, mask_comp, A, B), part, Sj, Sx, scap, T.p, T.j, (Z *)T.x, ccap, tot);
     prof_end(ps, s);
     long long h[3] = {0, 0, 0};
     const cudaError_t e = readback(h, tot, sizeof(h), s);
     if (e != cudaSuccess) { dev_free(T, s); return cuda_to_info(e); }
     if (h[2] != 0 || h[1] != SMALL_DONE) { dev_free(T, s); return NO_VALUE; }
     T.nnz = h[0];
+    if (ccap > 2 * T.nnz + (1 << 20)) trim_entries(T, sizeof(Z), s);
     C = T;
     return SUCCESS;
 }
@@ -2240,17 +2427,7 @@ static int saxpy3_t(DevCSR &C, const DevCSR *M, bool mask_comp, const DevCSR &A,
         }
         exec_pack<Z>(P, T.j, (Z *)T.x, s);
     } else if (cap > 2 * nnz + (1 << 20)) {
-        // far more room than entries: exact arrays
-        int32_t *j2 = (int32_t *)dalloc((size_t)(nnz + 1) * 4, s);
-        void *x2 = dalloc((size_t)(nnz + 1) * sizeof(Z), s);
-        if (j2 && x2) {
-            cudaMemcpyAsync(j2, T.j, (size_t)nnz * 4, cudaMemcpyDeviceToDevice, s);
-            cudaMemcpyAsync(x2, T.x, (size_t)nnz * sizeof(Z), cudaMemcpyDeviceToDevice, s);
-            dfree(T.j, s); dfree(T.x, s);
-            T.j = j2; T.x = x2;
-        } else {
-            dfree(j2, s); dfree(x2, s);
-        }
+        trim_entries(T, sizeof(Z), s);
     }
     info = cuda_to_info(cudaGetLastError());
     if (info != SUCCESS) { dev_free(T, s); return info; }
