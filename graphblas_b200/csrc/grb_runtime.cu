@@ -342,11 +342,12 @@ struct ReadbackBuffer {
     }
 };
 
-cudaError_t readback(void *dst, const void *src, size_t bytes, cudaStream_t s)
+// the calling thread's page, made on its first use; false where it cannot be
+static bool own_page(ReadbackPage *out)
 {
     thread_local ReadbackBuffer rb;
     ReadbackPage &pg = rb.pg;
-    if (!pg.host && bytes <= READBACK_MAX) {
+    if (!pg.host) {
         {
             std::lock_guard<std::mutex> lk(g_rb_mu);
             if (!g_rb_pool.empty()) {
@@ -368,6 +369,23 @@ cudaError_t readback(void *dst, const void *src, size_t bytes, cudaStream_t s)
             }
         }
     }
+    *out = pg;
+    return pg.host != nullptr;
+}
+
+bool readback_page(void **host, void **dev)
+{
+    ReadbackPage pg;
+    if (!own_page(&pg)) return false;
+    *host = pg.host;
+    *dev = pg.dev;
+    return true;
+}
+
+cudaError_t readback(void *dst, const void *src, size_t bytes, cudaStream_t s)
+{
+    ReadbackPage pg;
+    if (bytes <= READBACK_MAX) own_page(&pg);
     // a copy refused at submission leaves nothing for the synchronise to
     // report, so its own status is checked first (the bytes are not read)
     if (!pg.host || bytes > READBACK_MAX) {

@@ -71,6 +71,11 @@ void stream_scratch_release(cudaStream_t s);
 // copy `bytes` (at most a few KB) from the device after the stream's work,
 // synchronising the stream; returns its error
 cudaError_t readback(void *dst, const void *src, size_t bytes, cudaStream_t s);
+// The calling thread's page-locked page (4 KB) as the host and the device see
+// it: a call's last kernel writes its result's size there, and the host reads
+// it after it has synchronised the stream (the page is the call's until it
+// returns).
+bool readback_page(void **host, void **dev);
 
 // host-side allocation fault injection (the reference's malloc_debug
 // counter, Source/global/GB_Global.c:83-93): when armed with n > 0, the n-th

@@ -795,7 +795,6 @@ static constexpr int SMALL_CAP = 256;              // products per row, at most
 static constexpr int SMALL_POSB = 8;               // log2(SMALL_CAP)
 static constexpr int SMALL_CHUNK = 128;            // rows per block, at most
 static constexpr int SMALL_ARENA = 6144;           // bytes of products a warp holds
-static constexpr int64_t SMALL_MIN_ROWS = 2;       // rows of a product, at least
 enum { SMALL_DONE = 0, SMALL_TOO_LONG = 1, SMALL_NO_ROOM = 3 };
 
 template <typename Z> __host__ __device__ constexpr int small_arena_entries()
@@ -1542,6 +1541,362 @@ k_dense_compact(const int32_t *__restrict__ rows, int cblocks, int64_t ncols,
 }
 
 // ---------------------------------------------------------------------------
+// one-row products (vxm), order-free monoids
+// ---------------------------------------------------------------------------
+
+// w = u'*A over a dense accumulator, in three launches:
+//
+//   prep      some blocks clear the accumulator and mark the mask, the others
+//             scan the lengths of the rows of B that u reads (look-back
+//             tiles): wp[e] = products before entry e, boff[e] = first entry
+//             of its row of B less wp[e], so product t of entry e is B's entry
+//             boff[e] + t
+//   products  every product over the grid, ROW_U steps of 32 at a time by a
+//             warp, so that ROW_U chains of dependent loads (row, B's column,
+//             accumulator) are in flight
+//   compact   the columns that hold a value, in order, straight into w
+//             (sized for every column), and their number into page-locked
+//             memory: one synchronisation and no other read
+//
+// The separate scan of w's one row offset, the read-back launch, the packing
+// from slots and a second synchronisation took 45 us of a 95 us step.
+//
+// The accumulator of a column is one word: the packed state and k of a max-k
+// ANY (PackedDense); for a floating MIN / MAX the value's bits in an order
+// that unsigned integers share (all ones / zero where there is none), so a
+// term is one atomicMin / atomicMax that no other thread can fail, where a
+// compare-and-swap loop on a hub's column retries (1191 us of a six-hop
+// shortest-path pass on 260 thousand vertices, 239 us so); otherwise a
+// value and a flag byte.
+template <class SR> struct RowAcc {
+    using Z = typename SR::z_t;
+    static constexpr bool packed = PackedDense<SR>::on;
+    static constexpr bool coded = !packed && std::is_floating_point<Z>::value &&
+                                  (SR::add_op == OP_MIN || SR::add_op == OP_MAX);
+    static constexpr bool is_min = SR::add_op == OP_MIN;
+    using C = typename std::conditional<sizeof(Z) == 4, uint32_t, unsigned long long>::type;
+    using W = typename std::conditional<packed, unsigned long long,
+              typename std::conditional<coded, C, Z>::type>::type;
+    // are the flag bytes used?
+    static constexpr bool flags(bool has_mask) { return !packed && (!coded || has_mask); }
+    __device__ __forceinline__ static W init()
+    {
+        if constexpr (packed) return 0;
+        else if constexpr (coded) return is_min ? ~(C)0 : (C)0;
+        else return dense_init<SR>();
+    }
+};
+
+// a float's bits so that unsigned order is the numbers' order
+__device__ __forceinline__ uint32_t ordered_bits(float v)
+{
+    const uint32_t u = __float_as_uint(v);
+    return u ^ ((uint32_t)((int32_t)u >> 31) | 0x80000000u);
+}
+__device__ __forceinline__ unsigned long long ordered_bits(double v)
+{
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+    return u ^ ((unsigned long long)((long long)u >> 63) | 0x8000000000000000ull);
+}
+__device__ __forceinline__ float from_ordered(uint32_t u)
+{
+    return __uint_as_float(u & 0x80000000u ? u ^ 0x80000000u : ~u);
+}
+__device__ __forceinline__ double from_ordered(unsigned long long u)
+{
+    return __longlong_as_double((long long)(u >> 63 ? u ^ 0x8000000000000000ull : ~u));
+}
+
+template <class SR>
+__global__ void __launch_bounds__(LB_THREADS)
+k_row_prep(int nprep, int64_t ncols, uint8_t *__restrict__ flag,
+           typename RowAcc<SR>::W *__restrict__ val, const int32_t *__restrict__ Mp,
+           const int32_t *__restrict__ Mj, bool has_mask, bool mask_comp, int64_t nu,
+           const int32_t *__restrict__ Aj, const int32_t *__restrict__ Bp,
+           int32_t *__restrict__ wp, int32_t *__restrict__ boff,
+           unsigned long long *__restrict__ ws, int *__restrict__ err)
+{
+    using A = RowAcc<SR>;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if ((int)blockIdx.x < nprep) {
+        // a range of columns: cleared, then the mask's entries in it marked,
+        // 1 = allowed (plain mask), 2 = forbidden (complement)
+        __shared__ int32_t s_lo, s_hi;
+        const int64_t per = ((ncols + nprep - 1) / nprep + 255) & ~(int64_t)255;
+        const int64_t c0 = (int64_t)blockIdx.x * per;
+        const int64_t c1 = c0 + per < ncols ? c0 + per : ncols;
+        if (c0 >= c1) return;
+        const bool fl = A::flags(has_mask);
+        for (int64_t j = c0 + tid; j < c1; j += blockDim.x) {
+            val[j] = A::init();
+            if (fl) flag[j] = 0;
+        }
+        if (!has_mask) return;
+        if (warp < 2) {
+            const int32_t r = warp_lower_bound(Mj, Mp[0], Mp[1], (int32_t)(warp ? c1 : c0), lane);
+            if (lane == 0) { if (warp == 0) s_lo = r; else s_hi = r; }
+        }
+        __syncthreads();
+        const uint8_t st = mask_comp ? 2 : 1;
+        for (int32_t pm = s_lo + tid; pm < s_hi; pm += blockDim.x) {
+            if constexpr (A::packed) val[Mj[pm]] = (unsigned long long)st << 32;
+            else flag[Mj[pm]] = st;
+        }
+        return;
+    }
+    __shared__ int s_tile;
+    __shared__ int32_t s_ex;
+    __shared__ int32_t warp_sums[LB_THREADS / 32];
+    unsigned long long *status = ws + 1;
+    if (tid == 0) s_tile = (int)atomicAdd(&ws[0], 1ull);
+    __syncthreads();
+    const int64_t tile = s_tile;
+    const int64_t base = tile * LB_TILE + (int64_t)warp * (32 * LB_ROWS) + lane;
+    int32_t v[LB_ROWS], b0[LB_ROWS];
+    #pragma unroll
+    for (int r = 0; r < LB_ROWS; r++) b0[r] = base + r * 32 < nu ? Aj[base + r * 32] : -1;
+    #pragma unroll
+    for (int r = 0; r < LB_ROWS; r++) {
+        const int32_t k = b0[r];
+        v[r] = 0;
+        if (k >= 0) { b0[r] = Bp[k]; v[r] = Bp[k + 1] - b0[r]; }
+    }
+    int32_t run = 0;
+    #pragma unroll
+    for (int r = 0; r < LB_ROWS; r++) {
+        int32_t x = v[r];
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        v[r] = run + x - v[r];
+        run += __shfl_sync(0xffffffffu, x, 31);
+    }
+    if (lane == 0) warp_sums[warp] = run;
+    __syncthreads();
+    if (warp == 0) {
+        int32_t x = lane < LB_THREADS / 32 ? warp_sums[lane] : 0;
+        const int32_t own = x;
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        const long long agg = __shfl_sync(0xffffffffu, x, 31);
+        if (lane < LB_THREADS / 32) warp_sums[lane] = x - own;
+        long long ex = 0;
+        if (tile == 0) {
+            if (lane == 0) atomicExch(&status[0], LB_INC | (unsigned long long)agg);
+        } else {
+            if (lane == 0) atomicExch(&status[tile], LB_AGG | (unsigned long long)agg);
+            ex = lb_lookback(status, tile, lane, err);
+            if (lane == 0)
+                atomicExch(&status[tile], LB_INC | ((unsigned long long)(ex + agg) & LB_VAL));
+        }
+        if (lane == 0) s_ex = (int32_t)ex;
+    }
+    __syncthreads();
+    const int32_t wbase = s_ex + warp_sums[warp];
+    #pragma unroll
+    for (int r = 0; r < LB_ROWS; r++) {
+        const int64_t e = base + r * 32;
+        if (e <= nu) {                           // wp[nu] = all products
+            wp[e] = wbase + v[r];
+            if (e < nu) boff[e] = b0[r] - (wbase + v[r]);
+        }
+    }
+}
+
+static constexpr int ROW_U = 4;
+
+template <class SR>
+__global__ void __launch_bounds__(256)
+k_row_products(int64_t nu, const int32_t *__restrict__ wp, const int32_t *__restrict__ boff,
+               const int32_t *__restrict__ Aj, const void *__restrict__ Ax, bool a_iso,
+               const int32_t *__restrict__ Bj, const void *__restrict__ Bx, bool b_iso,
+               bool has_mask, bool mask_comp, uint8_t *__restrict__ flag,
+               typename RowAcc<SR>::W *__restrict__ val)
+{
+    using Z = typename SR::z_t;
+    using A = RowAcc<SR>;
+    using W = typename A::W;
+    constexpr bool idem = SR::M::any || SR::add_op == OP_MIN || SR::add_op == OP_MAX ||
+                          SR::add_op == OP_LOR || SR::add_op == OP_LAND;
+    const int lane = threadIdx.x & 31;
+    const int32_t total = wp[nu];
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    // spans of consecutive products, about four a warp, 128 to 1024 long: one
+    // search for the entry of a span's first product, and every later step
+    // goes on from the entry before
+    constexpr int STEP = 32 * ROW_U;
+    int64_t span = ((int64_t)total + 4 * nw - 1) / (4 * nw);
+    span = (span + STEP - 1) / STEP * STEP;
+    span = span < STEP ? STEP : (span > 1024 ? 1024 : span);
+    const int64_t nspan = ((int64_t)total + span - 1) / span;
+    for (int64_t si = wid; si < nspan; si += nw) {
+        // from the last span down: the first warps carry the largest k, so
+        // that a max-k ANY skips most later atomics; the result does not
+        // depend on the order
+        const int32_t s0 = (int32_t)((nspan - 1 - si) * span);
+        const int32_t s1 = (int64_t)s0 + span < total ? (int32_t)(s0 + span) : total;
+        int32_t e0 = warp_last_le<int32_t, int32_t>(wp, (int32_t)nu, s0, lane);
+        for (int32_t base = s0; base < s1; base += STEP) {
+            int32_t e[ROW_U], j[ROW_U], k[ROW_U], pb[ROW_U];
+            #pragma unroll
+            for (int u = 0; u < ROW_U; u++) {
+                const int32_t t = base + u * 32 + lane;
+                e[u] = warp_rows<int32_t, int32_t>(wp, (int32_t)nu, e0, t < s1 ? t : s1 - 1, lane);
+                e0 = __shfl_sync(0xffffffffu, e[u], 31);
+            }
+            #pragma unroll
+            for (int u = 0; u < ROW_U; u++) {
+                const int32_t t = base + u * 32 + lane;
+                k[u] = Aj[e[u]];
+                pb[u] = boff[e[u]] + t;
+                j[u] = t < s1 ? Bj[pb[u]] : -1;
+            }
+            W cur[ROW_U];
+            uint8_t f[ROW_U];
+            #pragma unroll
+            for (int u = 0; u < ROW_U; u++) {
+                f[u] = 0;
+                if (j[u] < 0) continue;
+                if (A::flags(has_mask)) f[u] = flag[j[u]];
+                if (A::packed || A::coded) cur[u] = val[j[u]];
+            }
+            #pragma unroll
+            for (int u = 0; u < ROW_U; u++) {
+                if (j[u] < 0) continue;
+                Z a = Z(), b = Z();
+                if constexpr (A::packed) {
+                    const unsigned st = (unsigned)(cur[u] >> 32);
+                    if (has_mask && (mask_comp ? st == 2 : st == 0)) continue;
+                    const Z tv = SR::F::f(a, b, 0, k[u], j[u]);
+                    const unsigned long long nv = PK_SET | (unsigned long long)(uint32_t)tv;
+                    if (cur[u] < nv) atomicMax(&val[j[u]], nv);
+                    continue;
+                }
+                if (has_mask && (mask_comp ? f[u] == 2 : f[u] == 0)) continue;
+                if (SR::needs_a) a = ld_val<Z>(Ax, e[u], a_iso);
+                if (SR::needs_b) b = ld_val<Z>(Bx, pb[u], b_iso);
+                Z tv = SR::F::f(a, b, 0, k[u], j[u]);
+                if constexpr (A::coded) {
+                    // a NaN loses to every number, as in the monoid's UPDATE,
+                    // and stays where there is none: its code lies between
+                    // the infinity that loses to every other number and the
+                    // code of no value
+                    if (isnan(tv)) tv = A::is_min ? (Z)NAN : -(Z)NAN;
+                    const typename A::C nv = ordered_bits(tv);
+                    if (A::is_min) { if (nv < cur[u]) atomicMin(&val[j[u]], nv); }
+                    else { if (nv > cur[u]) atomicMax(&val[j[u]], nv); }
+                } else if constexpr (!A::packed) {
+                    if constexpr (idem) {
+                        if (f[u] == 3) {
+                            if (SR::any_const) continue;
+                            const Z c = val[j[u]];
+                            if (SR::M::any ? !(tv > c) : (SR::M::update(c, tv) == c)) continue;
+                        }
+                    }
+                    AtomicUpd<SR::add_op, Z>::run(&val[j[u]], tv);
+                    if (f[u] != 3) flag[j[u]] = 3;
+                }
+            }
+        }
+    }
+}
+
+// tiles of 4096 columns from a ticket; a warp owns 512 of them, 32 at a time
+template <class SR>
+__global__ void __launch_bounds__(DG_THREADS)
+k_row_compact(int64_t ncols, const uint8_t *__restrict__ flag,
+              const typename RowAcc<SR>::W *__restrict__ val, int32_t *__restrict__ Wp,
+              int32_t *__restrict__ Wj, typename SR::z_t *__restrict__ Wx, int64_t ntiles,
+              unsigned long long *__restrict__ ws, int *__restrict__ err,
+              long long *__restrict__ host)
+{
+    using A = RowAcc<SR>;
+    using Z = typename SR::z_t;
+    using W = typename A::W;
+    __shared__ int s_tile;
+    __shared__ long long s_ex;
+    __shared__ int s_w[DG_THREADS / 32];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    unsigned long long *status = ws + 1;
+    if (tid == 0) s_tile = (int)atomicAdd(&ws[0], 1ull);
+    __syncthreads();
+    const int64_t tile = s_tile;
+    const int64_t c0 = tile * DG_CHUNK + w * (32 * DG_ITEMS) + lane;
+    W v[DG_ITEMS];
+    unsigned m[DG_ITEMS];
+    int run = 0;
+    #pragma unroll
+    for (int r = 0; r < DG_ITEMS; r++) {
+        const int64_t j = c0 + r * 32;
+        bool on = false;
+        if (j < ncols) {
+            if constexpr (A::packed) { v[r] = val[j]; on = (v[r] >> 32) == 3; }
+            else if constexpr (A::coded) { v[r] = val[j]; on = v[r] != A::init(); }
+            else on = flag[j] == 3;
+        }
+        m[r] = on;
+    }
+    #pragma unroll
+    for (int r = 0; r < DG_ITEMS; r++) {
+        m[r] = __ballot_sync(0xffffffffu, m[r] != 0);
+        run += __popc(m[r]);
+    }
+    if (lane == 0) s_w[w] = run;
+    __syncthreads();
+    if (w == 0) {
+        int x = lane < DG_THREADS / 32 ? s_w[lane] : 0;
+        const int own = x;
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        const long long agg = __shfl_sync(0xffffffffu, x, 31);
+        if (lane < DG_THREADS / 32) s_w[lane] = x - own;
+        long long ex = 0;
+        if (tile == 0) {
+            if (lane == 0) atomicExch(&status[0], LB_INC | (unsigned long long)agg);
+        } else {
+            if (lane == 0) atomicExch(&status[tile], LB_AGG | (unsigned long long)agg);
+            ex = lb_lookback(status, tile, lane, err);
+            if (lane == 0)
+                atomicExch(&status[tile], LB_INC | ((unsigned long long)(ex + agg) & LB_VAL));
+        }
+        if (lane == 0) {
+            s_ex = ex;
+            if (tile == ntiles - 1) {
+                Wp[0] = 0;
+                Wp[1] = (int32_t)(ex + agg);
+                // an error of this tile's own wait, or of any before it
+                host[0] = ex + agg;
+                host[1] = *(volatile int *)err;
+                __threadfence_system();
+            }
+        }
+    }
+    __syncthreads();
+    int64_t pos = s_ex + s_w[w];
+    const unsigned below = (1u << lane) - 1u;
+    #pragma unroll
+    for (int r = 0; r < DG_ITEMS; r++) {
+        if ((m[r] >> lane) & 1u) {
+            const int64_t j = c0 + r * 32, q = pos + __popc(m[r] & below);
+            Wj[q] = (int32_t)j;
+            if constexpr (A::packed) Wx[q] = (Z)(uint32_t)(v[r] & 0xffffffffull);
+            else if constexpr (A::coded) Wx[q] = from_ordered(v[r]);
+            else Wx[q] = val[j];
+        }
+        pos += __popc(m[r]);
+    }
+}
+
+// ---------------------------------------------------------------------------
 // phase 4: pack each row's (sorted) slot into CSR
 // ---------------------------------------------------------------------------
 
@@ -2163,86 +2518,6 @@ struct SlotSource {
     }
 };
 
-// A one-row product whose row is expected to be heavy (vxm with a large
-// frontier), with an order-free monoid: straight to the dense accumulator,
-// with no symbolic phase and no host round trip before it.  The row's A
-// entries are its whole flat index; its slots hold every column.
-template <class SR>
-static int saxpy3_row_dense(DevCSR &C, const DevCSR *M, bool mask_comp, const DevCSR &A,
-                            const DevCSR &B, SemiringCode sr, cudaStream_t s)
-{
-    using Z = typename SR::z_t;
-    const int64_t ncols = B.ncols;
-    SaxpyPlan *P = new SaxpyPlan();
-    struct PlanGuard { SaxpyPlan *P; cudaStream_t s; ~PlanGuard() { saxpy_plan_free(P, s); } }
-        pg{P, s};
-    P->sr = sr;
-    P->cfg = saxpy_default_config();
-    P->zsize = sizeof(Z);
-    P->order_free = true;
-    P->m = 1; P->ncols = ncols;
-    P->has_mask = M != nullptr; P->mask_comp = mask_comp;
-    const int nb = P->cfg.nb;
-    P->h_bins[nb + 1] = 1;
-    P->h_start[nb + 1] = 0;
-    P->heavy_alen = A.nnz;
-    P->heavy_chunk = 1;
-    P->total_cap = ncols;
-    const int64_t ntiles = (ncols + dense_tile<SR>() - 1) / dense_tile<SR>();
-    // everything in one allocation; the counters, the look-back workspaces,
-    // the slot offset, the row count and the row list (row 0) are zero
-    Carve cv(s);
-    auto layout = [&]() {
-        P->bins = cv.take<int>(BINS_WORDS);
-        P->lb_row = cv.take<unsigned long long>(scan_lb_ws_elems(2));
-        P->slot_off = cv.take<int64_t>(2);
-        P->row_cnt = cv.take<int32_t>(2);
-        P->bin_rows = cv.take<int32_t>(2);
-        P->lb_w = cv.take<unsigned long long>(lb_ws_elems(A.nnz + 1));
-        P->lb_c = cv.take<unsigned long long>(ntiles + 2);
-        P->Cp64 = cv.take<int64_t>(3);
-        P->hoff = cv.take<int64_t>(2);
-        P->hlen = cv.take<int64_t>(2);
-        P->hw_ws = cv.take<int64_t>(scan_ws_elems(2));
-        P->wprefix = cv.take<int64_t>(A.nnz + 1);
-        P->flag8 = cv.take<uint8_t>(ncols + 1);
-        P->val = cv.take<dense_val_t<SR>>(ncols + 1);
-    };
-    layout();
-    if (!cv.alloc()) return OUT_OF_MEMORY;
-    layout();
-    P->block = cv.base;
-    P->row_bin = nullptr;                 // the one row counts
-    cudaMemsetAsync(P->bins, 0, (size_t)((char *)(P->lb_c + ntiles + 2) - (char *)P->bins), s);
-    DevCSR T;
-    T.nrows = 1; T.ncols = ncols; T.type = sr.type; T.iso = false;
-    T.p = (int32_t *)dalloc(2 * 4, s);
-    if (!T.p) return OUT_OF_MEMORY;
-    SlotSource src(s);
-    void *slots = src.get(src.have >= slot_bytes(P, ncols) ? src.have : slot_bytes(P, ncols));
-    if (!slots) { dev_free(T, s); return OUT_OF_MEMORY; }
-    plan_place_slots(P, slots, src.have);
-    const int ps = prof_begin("saxpy3_numeric", s);
-    exec_heavy<SR>(P, M, A, B, s);
-    prof_end(ps, s);
-    exec_counts(P, T.p, nullptr, s);
-    int hb[BINS_READ];
-    cudaError_t e = readback(hb, P->bins, sizeof(hb), s);
-    if (e != cudaSuccess) { dev_free(T, s); return cuda_to_info(e); }
-    if (hb[BIN_ROW_ERR] || hb[BIN_HEAVY_ERR]) { dev_free(T, s); return PANIC; }
-    int64_t nnz = 0;
-    memcpy(&nnz, hb + BIN_NNZ, 8);
-    T.nnz = nnz;
-    T.j = (int32_t *)dalloc((size_t)(nnz + 1) * 4, s);
-    T.x = dalloc((size_t)(nnz + 1) * sizeof(Z), s);
-    if (!T.j || !T.x) { dev_free(T, s); return OUT_OF_MEMORY; }
-    exec_pack<Z>(P, T.j, (Z *)T.x, s);
-    const int info = cuda_to_info(cudaGetLastError());
-    if (info != SUCCESS) { dev_free(T, s); return info; }
-    C = T;
-    return SUCCESS;
-}
-
 // far more room than entries: exact arrays
 static void trim_entries(DevCSR &T, size_t zsize, cudaStream_t s)
 {
@@ -2253,6 +2528,81 @@ static void trim_entries(DevCSR &T, size_t zsize, cudaStream_t s)
     cudaMemcpyAsync(x, T.x, (size_t)T.nnz * zsize, cudaMemcpyDeviceToDevice, s);
     dfree(T.j, s); dfree(T.x, s);
     T.j = j; T.x = x;
+}
+
+// Which one-row products take the dense accumulator: those expected far past
+// the shared-memory bins, and any whose accumulator is small enough to clear
+// and read for less than the general path's launches cost (32 MB, about 10
+// us of HBM time, against ten launches and a second read, about 60 us).
+static constexpr int64_t ROW_CLEAR = (int64_t)32 << 20;
+
+// A one-row product with an order-free monoid (vxm): see k_row_prep.
+// NO_VALUE when w's arrays, sized for every column, cannot be had.
+template <class SR>
+static int saxpy3_row(DevCSR &C, const DevCSR *M, bool mask_comp, const DevCSR &A,
+                      const DevCSR &B, SemiringCode sr, double est, cudaStream_t s)
+{
+    using Z = typename SR::z_t;
+    using W = typename RowAcc<SR>::W;
+    const int64_t ncols = B.ncols, nu = A.nnz;
+    const int64_t tiles_u = (nu + 1 + LB_TILE - 1) / LB_TILE;
+    const int64_t tiles_c = (ncols + DG_CHUNK - 1) / DG_CHUNK;
+    void *host = nullptr, *host_dev = nullptr;
+    if (!readback_page(&host, &host_dev)) return NO_VALUE;
+    DevCSR T;
+    T.nrows = 1; T.ncols = ncols; T.type = sr.type; T.iso = false;
+    T.p = (int32_t *)dalloc(2 * 4, s);
+    if (!T.p) return OUT_OF_MEMORY;
+    T.j = (int32_t *)dalloc((size_t)(ncols + 1) * 4, s);
+    T.x = dalloc((size_t)(ncols + 1) * sizeof(Z), s);
+    // the error word and the look-back words of both scans first: one memset
+    int *err = nullptr;
+    unsigned long long *wsu = nullptr, *wsc = nullptr;
+    int32_t *wp = nullptr, *boff = nullptr;
+    uint8_t *flag = nullptr;
+    W *val = nullptr;
+    const bool fl = RowAcc<SR>::flags(M != nullptr);
+    Carve cv(s);
+    auto layout = [&]() {
+        err = cv.take<int>(1);
+        wsu = cv.take<unsigned long long>(tiles_u + 1);
+        wsc = cv.take<unsigned long long>(tiles_c + 1);
+        wp = cv.take<int32_t>(nu + 1);
+        boff = cv.take<int32_t>(nu + 1);
+        if (fl) flag = cv.take<uint8_t>(ncols);
+        val = cv.take<W>(ncols);
+    };
+    layout();
+    CallBlock blk(s);
+    const bool got = T.j && T.x && blk.get(cv.off);
+    if (!got) { dev_free(T, s); return NO_VALUE; }
+    cv.base = blk.base;
+    cv.off = 0;
+    layout();
+    cudaMemsetAsync(err, 0, (size_t)((char *)(wsc + tiles_c + 1) - (char *)err), s);
+    const int nprep = nblocks(ncols, 1024, 4);
+    k_row_prep<SR><<<(unsigned)(nprep + tiles_u), LB_THREADS, 0, s>>>(nprep, ncols, flag, val,
+        M ? M->p : nullptr, M ? M->j : nullptr, M != nullptr, mask_comp, nu, A.j, B.p, wp, boff,
+        wsu, err);
+    // as many warps as the expected products need, from one block per SM up
+    int64_t blocks = (int64_t)(est / 256.0) + 1;
+    const int64_t nsm = runtime().num_sms;
+    blocks = blocks < nsm ? nsm : blocks > nsm * 32 ? nsm * 32 : blocks;
+    const int ps = prof_begin("saxpy3_numeric", s);
+    k_row_products<SR><<<(unsigned)blocks, 256, 0, s>>>(nu, wp, boff, A.j, A.x, A.iso, B.j, B.x,
+        B.iso, M != nullptr, mask_comp, flag, val);
+    prof_end(ps, s);
+    k_row_compact<SR><<<(unsigned)tiles_c, DG_THREADS, 0, s>>>(ncols, flag, val, T.p, T.j,
+        (Z *)T.x, tiles_c, wsc, err, (long long *)host_dev);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) { dev_free(T, s); return cuda_to_info(e); }
+    const volatile long long *h = (const volatile long long *)host;
+    if (h[1]) { dev_free(T, s); return PANIC; }
+    T.nnz = h[0];
+    if (ncols > 2 * T.nnz + (1 << 22)) trim_entries(T, sizeof(Z), s);
+    C = T;
+    return SUCCESS;
 }
 
 // One-shot C<M> = A*B with one host round trip in the common case.  The
@@ -2279,7 +2629,7 @@ static int saxpy3_small(DevCSR &C, const DevCSR *M, bool mask_comp, const DevCSR
 {
     using Z = typename SR::z_t;
     const int64_t m = A.nrows;
-    if (m < SMALL_MIN_ROWS || A.nnz <= 0 || B.ncols >= ((int64_t)1 << 24)) return NO_VALUE;
+    if (A.nnz <= 0 || B.ncols >= ((int64_t)1 << 24)) return NO_VALUE;
     const double mean_b = B.nrows > 0 ? (double)B.nnz / (double)B.nrows : 0.0;
     const double flops_est = (double)A.nnz * (mean_b > 1.0 ? mean_b : 1.0);
     if (flops_est > 0.5 * SMALL_CAP * (double)m) return NO_VALUE;
@@ -2335,13 +2685,15 @@ static int saxpy3_t(DevCSR &C, const DevCSR *M, bool mask_comp, const DevCSR &A,
     const int64_t m = A.nrows;
     const double mean_b = B.nrows > 0 ? (double)B.nnz / (double)B.nrows : 0.0;
     if constexpr (SR::order_free) {
-        // a one-row product expected far past the shared-memory bins, whose
-        // dense row fits comfortably: the dense path directly
-        const SaxpyConfig dc = saxpy_default_config();
         const double est = (double)A.nnz * mean_b;
-        if (m == 1 && A.nnz > 0 && est >= 2.0 * (double)dc.bin[dc.nb - 1].limit &&
-            (double)B.ncols * (1.0 + sizeof(Z)) <= (double)((int64_t)4 << 30))
-            return saxpy3_row_dense<SR>(C, M, mask_comp, A, B, sr, s);
+        const SaxpyConfig dc = saxpy_default_config();
+        const double words = (double)B.ncols * (1.0 + sizeof(typename RowAcc<SR>::W));
+        if (m == 1 && A.nnz > 0 && B.ncols > 0 && words <= (double)((int64_t)4 << 30) &&
+            (words <= (double)ROW_CLEAR ||
+             est >= 2.0 * (double)dc.bin[dc.nb - 1].limit)) {
+            const int r = saxpy3_row<SR>(C, M, mask_comp, A, B, sr, est, s);
+            if (r != NO_VALUE) return r;
+        }
     }
     {
         const int r = saxpy3_small<SR>(C, M, mask_comp, A, B, sr, s);
