@@ -169,9 +169,11 @@ static inline int grid_n(int64_t n, int threads = 256)
 
 // ---------------------------------------------------------------------------
 // one-row union: w<u> = u with u's pattern as the structural mask, no
-// accumulator, no replace (the BFS parent update) on row vectors.  The
-// result is the merge of two sorted index lists in which u's entry wins a
-// tie.  One launch: tiles of UN_TILE merged positions (from a ticket); a
+// accumulator, no replace (the BFS parent update), and w = accum(w, u) with
+// no mask (a shortest-path step) on row vectors.  The result is the merge of
+// two sorted index lists in which u's entry wins a tie, or the accumulator
+// combines the two.  One launch (the accumulator's general form takes nine,
+// 65 us of a step on small vectors): tiles of UN_TILE merged positions (from a ticket); a
 // tile finds where its positions start in each list (merge path: a
 // warp-cooperative search over the diagonal), stages both ranges in shared
 // memory, each thread merges UN_ITEMS positions, the tile's kept count gets
@@ -207,15 +209,15 @@ __device__ __forceinline__ int64_t union_split(const int32_t *__restrict__ C, in
     return lo;
 }
 
-template <typename Z>
+template <typename Z, bool ACC>
 __global__ void __launch_bounds__(UN_THREADS)
 k_union_row(const int32_t *__restrict__ Cj, const Z *__restrict__ Cx, bool c_iso, int64_t nC,
             const int32_t *__restrict__ Tj, const Z *__restrict__ Tx, bool t_iso, int64_t nT,
-            int32_t *__restrict__ Rp, int32_t *__restrict__ Rj, Z *__restrict__ Rx,
-            int64_t *__restrict__ total, int64_t ntiles, unsigned long long *__restrict__ ws,
-            int *__restrict__ err)
+            int accum, int32_t *__restrict__ Rp, int32_t *__restrict__ Rj, Z *__restrict__ Rx,
+            int64_t ntiles, unsigned long long *__restrict__ ws, int *__restrict__ err,
+            long long *__restrict__ host)
 {
-    __shared__ int s_tile, s_last, s_agg;
+    __shared__ int s_tile, s_agg;
     __shared__ long long s_ex;
     __shared__ int64_t s_i0, s_i1;
     __shared__ int s_w[UN_THREADS / 32];
@@ -225,8 +227,10 @@ k_union_row(const int32_t *__restrict__ Cj, const Z *__restrict__ Cx, bool c_iso
     __shared__ __align__(16) int32_t s_buf[2 * UN_TILE];
     int32_t *s_c = s_buf, *s_t = s_buf + UN_TILE;
     int32_t *s_oj = s_buf, *s_os = s_buf + UN_TILE;
+    // with an accumulator: the entry of C that an entry of T meets, or -1
+    __shared__ int32_t s_oc[ACC ? UN_TILE : 1];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    unsigned long long *status = ws + 2;
+    unsigned long long *status = ws + 1;
     if (tid == 0) s_tile = (int)atomicAdd(&ws[0], 1ull);
     __syncthreads();
     const int64_t tile = s_tile;
@@ -246,6 +250,7 @@ k_union_row(const int32_t *__restrict__ Cj, const Z *__restrict__ Cx, bool c_iso
     for (int k = tid; k < nc; k += UN_THREADS) s_c[k] = Cj[i0 + k];
     for (int k = tid; k < nt; k += UN_THREADS) s_t[k] = Tj[j0 + k];
     const int32_t tprev = j0 > 0 ? Tj[j0 - 1] : -1;     // the T entry before the tile's
+    const int32_t cnext = ACC && i1 < nC ? Cj[i1] : -1; // the C entry after the tile's
     __syncthreads();
     // this thread's positions [dl, dl + UN_ITEMS) of the tile, merged locally
     const int dl = tid * UN_ITEMS;
@@ -261,12 +266,13 @@ k_union_row(const int32_t *__restrict__ Cj, const Z *__restrict__ Cx, bool c_iso
         ci = lo;
         tj = dl - lo;
     }
-    int32_t oj[UN_ITEMS], os[UN_ITEMS];
+    int32_t oj[UN_ITEMS], os[UN_ITEMS], oc[UN_ITEMS];
     int kept = 0;
     for (int k = 0; k < UN_ITEMS && dl + k < nl; k++) {
         if (tj < nt && (ci >= nc || s_t[tj] <= s_c[ci])) {
             oj[kept] = s_t[tj];
             os[kept] = (int32_t)(0x80000000u | (uint32_t)tj);
+            if (ACC) oc[kept] = (ci < nc ? s_c[ci] : cnext) == s_t[tj] ? ci : -1;
             kept++;
             tj++;
         } else {
@@ -309,13 +315,22 @@ k_union_row(const int32_t *__restrict__ Cj, const Z *__restrict__ Cx, bool c_iso
             s_ex = ex;
             s_agg = (int)agg;
             if (tile == 0) Rp[0] = 0;
-            if (tile == ntiles - 1) { Rp[1] = (int32_t)(ex + agg); *total = ex + agg; }
+            if (tile == ntiles - 1) {
+                Rp[1] = (int32_t)(ex + agg);
+                host[0] = ex + agg;
+                host[1] = *(volatile int *)err;
+                __threadfence_system();
+            }
         }
     }
     // (the block barrier above also ends every read of the staged inputs)
     __syncthreads();
     int loc = s_w[w] + (x - kept);
-    for (int k = 0; k < kept; k++) { s_oj[loc + k] = oj[k]; s_os[loc + k] = os[k]; }
+    for (int k = 0; k < kept; k++) {
+        s_oj[loc + k] = oj[k];
+        s_os[loc + k] = os[k];
+        if (ACC) s_oc[loc + k] = os[k] < 0 ? oc[k] : -1;
+    }
     __syncthreads();
     const int64_t base = s_ex;
     const int agg = s_agg;
@@ -328,6 +343,8 @@ k_union_row(const int32_t *__restrict__ Cj, const Z *__restrict__ Cx, bool c_iso
         if (k < agg) {
             const int32_t src = s_os[k];
             v[r] = src < 0 ? Tx[t_iso ? 0 : j0 + (src & 0x7fffffff)] : Cx[c_iso ? 0 : i0 + src];
+            if (ACC && s_oc[k] >= 0)
+                v[r] = apply_accum<Z>(accum, Cx[c_iso ? 0 : i0 + s_oc[k]], v[r]);
         }
     }
     #pragma unroll
@@ -338,56 +355,55 @@ k_union_row(const int32_t *__restrict__ Cj, const Z *__restrict__ Cx, bool c_iso
             Rx[base + k] = v[r];
         }
     }
-    // the last tile to finish clears the workspace
-    if (tid == 0) {
-        __threadfence();
-        s_last = atomicAdd(&ws[1], 1ull) == (unsigned long long)(ntiles - 1);
-    }
-    __syncthreads();
-    if (s_last) {
-        for (int64_t t = tid; t < ntiles; t += UN_THREADS) status[t] = 0;
-        if (tid == 0) { ws[0] = 0; ws[1] = 0; }
-    }
 }
 
-// C = C union T on one row, T's entries winning ties (w<u> = u)
+// C = C union T on one row, T's entries winning ties (w<u> = u), or combined
+// with C's by the accumulator
 template <typename Z>
-static int union_row_t(DevCSR &C, const DevCSR &T, cudaStream_t s)
+static int union_row_t(DevCSR &C, const DevCSR &T, int accum, cudaStream_t s)
 {
     const int64_t nC = C.nnz, nT = T.nnz, nd = nC + nT;
     if (nd >= INT32_MAX) return OUT_OF_MEMORY;
     const int64_t ntiles = nd > 0 ? (nd + UN_TILE - 1) / UN_TILE : 0;
+    void *host = nullptr, *host_dev = nullptr;
+    if (!readback_page(&host, &host_dev)) return OUT_OF_MEMORY;
     Carve cv(s);
-    int64_t *tot_d = nullptr;
+    int *err = nullptr;
     unsigned long long *ws = nullptr;
     auto layout = [&]() {
-        tot_d = cv.take<int64_t>(2);
-        ws = cv.take<unsigned long long>(ntiles + 2);
+        err = cv.take<int>(1);
+        ws = cv.take<unsigned long long>(ntiles + 1);
     };
     layout();
-    if (!cv.alloc()) return OUT_OF_MEMORY;
+    CallBlock blk(s);
+    if (!blk.get(cv.off)) return OUT_OF_MEMORY;
+    cv.base = blk.base;
+    cv.off = 0;
     layout();
-    struct Release { Carve &c; ~Release() { dfree(c.base, c.s); } } release{cv};
     DevCSR R;
     R.nrows = 1; R.ncols = T.ncols; R.type = T.type; R.iso = false;
     R.p = (int32_t *)dalloc(2 * 4, s);
     R.j = (int32_t *)dalloc((size_t)(nd ? nd : 1) * 4, s);
     R.x = dalloc((size_t)(nd ? nd : 1) * sizeof(Z), s);
     if (!R.p || !R.j || !R.x) { dev_free(R, s); return OUT_OF_MEMORY; }
-    int64_t tot[2] = {0, 0};
+    R.nnz = 0;
     if (ntiles > 0) {
-        cudaMemsetAsync(tot_d, 0, (size_t)((char *)(ws + ntiles + 2) - (char *)tot_d), s);
-        k_union_row<Z><<<(unsigned)ntiles, UN_THREADS, 0, s>>>(C.j, (const Z *)C.x, C.iso, nC,
-            T.j, (const Z *)T.x, T.iso, nT, R.p, R.j, (Z *)R.x, tot_d, ntiles, ws,
-            (int *)(tot_d + 1));
-        cudaError_t e = readback(tot, tot_d, 16, s);
-        if (e == cudaSuccess) e = cudaGetLastError();
+        cudaMemsetAsync(err, 0, (size_t)((char *)(ws + ntiles + 1) - (char *)err), s);
+        auto launch = [&](auto kernel) {
+            kernel<<<(unsigned)ntiles, UN_THREADS, 0, s>>>(C.j, (const Z *)C.x, C.iso, nC,
+                T.j, (const Z *)T.x, T.iso, nT, accum, R.p, R.j, (Z *)R.x, ntiles, ws, err,
+                (long long *)host_dev);
+        };
+        if (accum) launch(k_union_row<Z, true>); else launch(k_union_row<Z, false>);
+        cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) { dev_free(R, s); return cuda_to_info(e); }
-        if ((int)tot[1] != 0) { dev_free(R, s); return PANIC; }
+        const volatile long long *h = (const volatile long long *)host;
+        if (h[1]) { dev_free(R, s); return PANIC; }
+        R.nnz = h[0];
     } else {
         cudaMemsetAsync(R.p, 0, 2 * 4, s);
     }
-    R.nnz = tot[0];
     dev_free(C, s);
     C = R;
     return SUCCESS;
@@ -399,7 +415,8 @@ static int accum_mask_t(DevCSR &C, const DevCSR &T, const DevCSR *M, bool comp,
 {
     const int64_t m = T.nrows, nT = T.nnz, nC = C.nnz;
     if (m == 1 && M && !comp && !replace && !accum && M->p == T.p && M->j == T.j)
-        return union_row_t<Z>(C, T, s);
+        return union_row_t<Z>(C, T, 0, s);
+    if (m == 1 && !M && !comp && accum) return union_row_t<Z>(C, T, accum, s);
     // the totals and error word, the two scans' workspaces, the keep flags /
     // offsets of both sides and T's values in one allocation; the first three
     // are cleared by one memset

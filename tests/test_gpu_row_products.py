@@ -1,0 +1,117 @@
+"""One-row products (vxm) with order-free monoids and the one-row write-back
+with an accumulator, at the edges of their tiles: 4096 columns of the dense
+accumulator, 2048 entries of u, 3072 merged positions.  Checked against the
+oracle."""
+
+import numpy as np
+import pytest
+
+from graphblas_b200 import workloads as W
+from tests.helpers import assert_exact, random_csr
+
+pytestmark = pytest.mark.gpu
+
+SEMIRINGS = [("MIN", "PLUS", "fp32", np.float32), ("MIN", "PLUS", "fp64", np.float64),
+             ("MAX", "PLUS", "fp32", np.float32), ("MIN", "PLUS", "int64", np.int64),
+             ("PLUS", "TIMES", "int32", np.int32), ("ANY", "SECONDI", "int64", np.int64),
+             ("ANY", "SECONDI", "int32", np.int32), ("ANY", "PAIR", "bool", np.bool_),
+             ("LOR", "LAND", "bool", np.bool_), ("MAX", "SECONDI", "int64", np.int64)]
+
+
+def row(n, nu, seed, dtype):
+    rng = np.random.default_rng(seed)
+    i = np.sort(rng.choice(n, nu, replace=False)).astype(np.int64)
+    x = (rng.random(nu) < 0.7) if dtype == np.bool_ else (rng.random(nu) * 20 - 10).astype(dtype)
+    return W.Csr(1, n, np.array([0, nu], np.int64), i, x)
+
+
+@pytest.fixture(scope="module")
+def operands():
+    """B per (rows, columns): some empty rows, one that spans most columns."""
+    made = {}
+
+    def get(k, n, dtype):
+        if (k, n) not in made:
+            B = random_csr(k, n, min(1.0, 6.0 / n), 11, np.float64, empty_rows=0.2)
+            hub = np.sort(np.random.default_rng(12).choice(n, max(1, n * 3 // 4), replace=False))
+            p = B.p.copy()
+            r = k // 2
+            old = slice(p[r], p[r + 1])
+            i = np.concatenate([B.i[:old.start], hub, B.i[old.stop:]]).astype(np.int64)
+            p[r + 1:] += len(hub) - (old.stop - old.start)
+            made[k, n] = (p, i)
+        p, i = made[k, n]
+        rng = np.random.default_rng(13)
+        x = (rng.random(len(i)) < 0.7) if dtype == np.bool_ else \
+            (rng.random(len(i)) * 20 - 10).astype(dtype)
+        return W.Csr(k, n, p, i, x)
+    return get
+
+
+@pytest.mark.parametrize("add,mult,tname,np_t", SEMIRINGS)
+@pytest.mark.parametrize("mask", [None, "plain", "complement"])
+@pytest.mark.parametrize("k,n,nu", [(40, 33, 1), (3000, 4096, 2047), (3000, 4097, 2048),
+                                    (2500, 9000, 2500)])
+def test_one_row_product(gpu, oracle, operands, add, mult, tname, np_t, mask, k, n, nu):
+    gb = gpu
+    tc = gb.TYPES[tname]
+    B = operands(k, n, np_t)
+    u = row(k, nu, 21, np_t)
+    M = row(n, max(1, n // 3), 22, np.bool_) if mask else None
+    if M:
+        M.x = None
+    dB, du = gb.DMatrix.upload(B, tname), gb.DMatrix.upload(u, tname)
+    dM = gb.DMatrix.upload(M, "bool") if M else None
+    C = gb.saxpy3(du, dB, gb.semiring(add, mult, tname), M=dM, mask_comp=mask == "complement")
+    got = C.download()
+    want = oracle.saxpy(1, n, (u.p, u.i, u.x, tc), (B.p, B.i, B.x, tc), add, mult, tc,
+                        M=(M.p, M.i, None, 1) if M else None, mask_comp=mask == "complement")
+    assert_exact(got, want, "%s_%s_%s" % (add, mult, tname))
+    for d in (dB, du, dM, C):
+        if d is not None:
+            d.free()
+
+
+@pytest.mark.parametrize("add,tname,np_t", [("MIN", "fp32", np.float32),
+                                            ("MIN", "fp64", np.float64),
+                                            ("MAX", "fp32", np.float32)])
+def test_one_row_product_nan_and_infinities(gpu, oracle, add, tname, np_t):
+    """A column of NaN alone is NaN, one NaN among numbers loses, infinities
+    are numbers."""
+    gb = gpu
+    tc = gb.TYPES[tname]
+    inf, nan = np.inf, np.nan
+    rows = [[nan, inf, -inf, 1.0, nan], [nan, inf, 5.0, nan, -2.0], [nan, 7.0, inf, -3.0, nan]]
+    p = np.arange(0, 16, 5).astype(np.int64)
+    i = np.tile(np.arange(5), 3).astype(np.int64)
+    B = W.Csr(3, 5, p, i, np.concatenate(rows).astype(np_t))
+    u = W.Csr(1, 3, np.array([0, 3], np.int64), np.arange(3, dtype=np.int64),
+              np.array([0.0, 1.0, 2.0], np_t))
+    dB, du = gb.DMatrix.upload(B), gb.DMatrix.upload(u)
+    C = gb.saxpy3(du, dB, gb.semiring(add, "PLUS", tname))
+    gp, gi, gx = C.download()
+    wp, wi, wx = oracle.saxpy(1, 5, (u.p, u.i, u.x, tc), (B.p, B.i, B.x, tc), add, "PLUS", tc)
+    assert np.array_equal(gp, wp) and np.array_equal(gi, wi)
+    assert np.array_equal(gx, wx, equal_nan=True)
+    for d in (dB, du, C):
+        d.free()
+
+
+@pytest.mark.parametrize("accum,op", [("GrB_MIN_FP32", "MIN"), ("GrB_PLUS_FP32", "PLUS"),
+                                      ("GrB_MINUS_FP32", "MINUS"), ("GrB_SECOND_FP32", "SECOND")])
+@pytest.mark.parametrize("nw,nu", [(0, 5), (7, 0), (1, 1), (1536, 1536), (3072, 1), (3073, 3000),
+                                   (4000, 9000)])
+def test_one_row_accumulate(gpu, oracle, accum, op, nw, nu):
+    """w = accum(w, u) without a mask, with entries of both in one tile and
+    equal entries on both sides of a tile's edge."""
+    from graphblas_b200.grb import API
+    api = API()
+    n = 9001
+    w, u = row(n, nw, 31, np.float32), row(n, nu, 32, np.float32)
+    hw, hu = (api.vector_from(v.i, v.x, 10, n) for v in (w, u))
+    api.assign_all(hw, None, accum, hu, n)
+    i, x = api.vector_to(hw, 10)
+    want = oracle.accum_mask(1, n, (w.p, w.i, w.x), (u.p, u.i, u.x), 10, accum=op)
+    assert_exact((np.array([0, len(i)]), i, x), want, op)
+    api.vfree(hw)
+    api.vfree(hu)
