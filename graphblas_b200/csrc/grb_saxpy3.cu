@@ -975,6 +975,246 @@ k_saxpy_small(int32_t m, int32_t chunk, EscIn in, long long *__restrict__ part,
 }
 
 // ---------------------------------------------------------------------------
+// phase 3a'': rows past the expand-sort-compress bin, dense in shared memory
+// ---------------------------------------------------------------------------
+
+// One block per row, the row dense in shared memory (a value and a bit per
+// column of C), its columns cut into TILE_T tiles of about as many entries of
+// B each.  A warp takes a few adjacent tiles at a time and streams all of the
+// row's products that fall in them, in ascending k, 32 at a time: no other
+// warp writes those columns, so nothing is synchronised inside the row, the
+// loads of four steps are in flight together, and two products of one column
+// in a step are found by a warp match and folded by the first of them in lane
+// order, which is k order.  Every column is folded in ascending k as in the
+// other kernels: the same bits for every semiring.  split[k][t] is where tile
+// t starts in row k of B.
+//
+// The kernels this replaces where C's rows fit (hash tables with one
+// synchronisation for each k, and dense rows in global memory by one block
+// with a dependent chain of five loads and a block barrier for each k) were
+// bound by latency: 2509 us for the 38M products (fp64) of the square of a
+// skewed graph of 5000 vertices, against 713 us.
+static constexpr int TILE_T = 32;                // tiles of a row, at most
+static constexpr int TILE_WARPS = 8;
+static constexpr int TILE_U = 4;                 // steps of 32 products in flight
+
+// entries of B in each column
+__global__ void k_tile_hist(const int32_t *__restrict__ Bj, int64_t nnz, int *__restrict__ hist)
+{
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nnz;
+         e += (int64_t)gridDim.x * blockDim.x)
+        atomicAdd(&hist[Bj[e]], 1);
+}
+
+// bound[t] = the first column that has t / TILE_T of B's entries before it
+__global__ void __launch_bounds__(1024)
+k_tile_bounds(const int *__restrict__ hist, int32_t ncols, int64_t nnz,
+              int32_t *__restrict__ bound)
+{
+    __shared__ long long s_w[32];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int32_t per = (ncols + 1023) / 1024;
+    const int32_t c0 = min(tid * per, ncols), c1 = min(c0 + per, ncols);
+    long long sum = 0;
+    for (int32_t c = c0; c < c1; c++) sum += hist[c];
+    long long x = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) s_w[w] = x;
+    if (tid <= TILE_T) bound[tid] = tid == 0 ? 0 : ncols;
+    __syncthreads();
+    long long ex = x - sum;
+    for (int q = 0; q < w; q++) ex += s_w[q];
+    auto tile_of = [&](long long before) {
+        const long long t = nnz > 0 ? before * TILE_T / nnz : 0;
+        return (int)(t < TILE_T - 1 ? t : TILE_T - 1);
+    };
+    // a column opens the tiles past the one before it
+    for (int32_t c = c0; c < c1; c++) {
+        const int t = tile_of(ex);
+        const int prev = c == 0 ? 0 : tile_of(ex - hist[c - 1]);
+        for (int q = prev + 1; q <= t; q++) bound[q] = c;
+        ex += hist[c];
+    }
+}
+
+__global__ void k_tile_split(const int32_t *__restrict__ Bp, const int32_t *__restrict__ Bj,
+                             int64_t nrows, const int32_t *__restrict__ bound,
+                             int32_t *__restrict__ split)
+{
+    const int64_t n = nrows * (TILE_T + 1);
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n;
+         q += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t k = q / (TILE_T + 1);
+        const int t = (int)(q - k * (TILE_T + 1));
+        const int32_t p0 = Bp[k], p1 = Bp[k + 1];
+        split[q] = t == 0 ? p0 : t == TILE_T ? p1 : lower_bound(Bj, p0, p1, bound[t]);
+    }
+}
+
+template <typename Z> static size_t tile_smem(int64_t ncols, bool has_mask)
+{
+    const size_t words = (size_t)((ncols + 31) / 32);
+    return (size_t)ncols * sizeof(Z) + 16 + words * 4 * (has_mask ? 2 : 1);
+}
+
+// rows of `rows`, from the last (the heaviest bin's) to the first
+template <class SR>
+__global__ void __launch_bounds__(TILE_WARPS * 32, 4)
+k_saxpy_tile(const int32_t *__restrict__ rows, int nrows, int *__restrict__ next, EscIn in,
+             const int32_t *__restrict__ split, int32_t ncols,
+             const int64_t *__restrict__ flops, const int64_t *__restrict__ slot_off,
+             int32_t *__restrict__ Tj, typename SR::z_t *__restrict__ Tx,
+             int32_t *__restrict__ row_cnt)
+{
+    using Z = typename SR::z_t;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ EscEnt<Z> s_ent[TILE_WARPS][ESC_ENTS];
+    __shared__ int s_row, s_group;
+    __shared__ int s_w[TILE_WARPS];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const unsigned upto = 0xffffffffu >> (31 - lane), below = upto >> 1;
+    Z *acc = (Z *)smem;
+    const int words = (ncols + 31) / 32;
+    uint32_t *bits = (uint32_t *)(smem + (((size_t)ncols * sizeof(Z) + 15) & ~(size_t)15));
+    uint32_t *mbits = bits + words;
+    EscEnt<Z> *ent = s_ent[w];
+    while (true) {
+        __syncthreads();
+        if (tid == 0) { s_row = atomicAdd(next, 1); s_group = 0; }
+        for (int q = tid; q < words; q += blockDim.x) {
+            bits[q] = 0;
+            if (in.has_mask) mbits[q] = 0;
+        }
+        __syncthreads();
+        if (s_row >= nrows) return;
+        const int32_t i = rows[nrows - 1 - s_row];
+        const int32_t pa0 = in.Ap[i], pa1 = in.Ap[i + 1];
+        if (in.has_mask) {
+            for (int32_t pm = in.Mp[i] + tid; pm < in.Mp[i + 1]; pm += blockDim.x)
+                atomicOr(&mbits[in.Mj[pm] >> 5], 1u << (in.Mj[pm] & 31));
+            __syncthreads();
+        }
+        // tiles that a warp takes at a time: a group of a short row holds a
+        // few hundred products too
+        const int64_t f = flops[i];
+        const int gs = f >= 16384 ? 1 : f >= 4096 ? 2 : 4;
+        while (true) {
+            int g = 0;
+            if (lane == 0) g = atomicAdd(&s_group, 1);
+            g = __shfl_sync(0xffffffffu, g, 0);
+            const int t0 = g * gs;
+            if (t0 >= TILE_T) break;
+            for (int32_t c0 = pa0; c0 < pa1; c0 += ESC_ENTS) {
+                const int32_t pa = c0 + lane;
+                int32_t k = 0, b0 = 0, len = 0;
+                Z a = Z();
+                if (pa < pa1) {
+                    k = in.Aj[pa];
+                    const int32_t *sp = split + (int64_t)k * (TILE_T + 1) + t0;
+                    b0 = sp[0];
+                    len = sp[gs] - b0;
+                    if (SR::needs_a) a = ld_val<Z>(in.Ax, pa, in.a_iso);
+                }
+                int incl = len;
+                #pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                const int total = __shfl_sync(0xffffffffu, incl, 31);
+                const int excl = incl - len;
+                const unsigned vm = __ballot_sync(0xffffffffu, len > 0);
+                __syncwarp();                    // the last chunk's entries are read
+                if (len > 0) ent[__popc(vm & below)] = EscEnt<Z>{b0 - excl, k, a};
+                __syncwarp();
+                int c = -1;
+                for (int q0 = 0; q0 < total; q0 += 32 * TILE_U) {
+                    int32_t j[TILE_U];
+                    int src[TILE_U];
+                    Z b[TILE_U];
+                    #pragma unroll
+                    for (int u = 0; u < TILE_U; u++) {
+                        const unsigned st = __reduce_or_sync(
+                            0xffffffffu, len > 0 && (excl >> 5) == (q0 >> 5) + u
+                                             ? 1u << (excl & 31) : 0u);
+                        src[u] = c + __popc(st & upto);
+                        c += __popc(st);
+                        const int q = q0 + u * 32 + lane;
+                        j[u] = -1;
+                        b[u] = Z();
+                        if (q < total) {
+                            const int32_t pb = ent[src[u]].base + q;
+                            j[u] = in.Bj[pb];
+                            if (SR::needs_b) b[u] = ld_val<Z>(in.Bx, pb, in.b_iso);
+                        }
+                    }
+                    #pragma unroll
+                    for (int u = 0; u < TILE_U; u++) {
+                        if (q0 + u * 32 >= total) break;
+                        bool valid = j[u] >= 0;
+                        if (in.has_mask && valid)
+                            valid = (((mbits[j[u] >> 5] >> (j[u] & 31)) & 1u) != 0) != in.mask_comp;
+                        Z z = Z();
+                        if (valid) {
+                            const EscEnt<Z> e = ent[src[u]];
+                            z = SR::F::f(e.a, b[u], i, e.k, j[u]);
+                        }
+                        const unsigned same =
+                            __match_any_sync(0xffffffffu, valid ? j[u] : -1 - lane);
+                        const bool first = valid && (same & below) == 0;
+                        unsigned rest = first ? same & ~upto : 0u;
+                        const Z own = z;
+                        bool was = false;
+                        if (first) {
+                            was = (bits[j[u] >> 5] >> (j[u] & 31)) & 1u;
+                            if (was) z = SR::M::update(acc[j[u]], z);
+                        }
+                        while (__any_sync(0xffffffffu, rest != 0)) {
+                            const Z t = shfl<Z>(own, rest ? __ffs(rest) - 1 : lane);
+                            if (rest) { z = SR::M::update(z, t); rest &= rest - 1; }
+                        }
+                        if (first) {
+                            acc[j[u]] = z;
+                            if (!was) atomicOr(&bits[j[u] >> 5], 1u << (j[u] & 31));
+                        }
+                        __syncwarp();
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        // the set columns in order: each warp a range of words
+        const int per = (words + TILE_WARPS - 1) / TILE_WARPS;
+        const int w0 = min(w * per, words), w1 = min(w0 + per, words);
+        int cnt = 0;
+        for (int q = w0 + lane; q < w1; q += 32) cnt += __popc(bits[q]);
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        if (lane == 0) s_w[w] = cnt;
+        __syncthreads();
+        int64_t pos = slot_off[i];
+        int all = 0;
+        #pragma unroll
+        for (int q = 0; q < TILE_WARPS; q++) {
+            if (q < w) pos += s_w[q];
+            all += s_w[q];
+        }
+        if (tid == 0) row_cnt[i] = all;
+        for (int q = w0; q < w1; q++) {
+            const uint32_t m = bits[q];
+            if ((m >> lane) & 1u) {
+                const int64_t at = pos + __popc(m & below);
+                Tj[at] = q * 32 + lane;
+                Tx[at] = acc[q * 32 + lane];
+            }
+            pos += __popc(m);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // phase 3b: heavy rows, dense accumulator in global memory
 // ---------------------------------------------------------------------------
 
@@ -2360,11 +2600,67 @@ static void launch_bin(const SaxpyPlan *P, int q, const DevCSR &A, const DevCSR 
 // m as every bin's bound and the fit check on the device
 template <class SR>
 static void exec_light(const SaxpyPlan *P, const DevCSR *M, const DevCSR &A, const DevCSR &B,
-                       bool exact, cudaStream_t s)
+                       bool exact, cudaStream_t s, int nbins = MAX_SMEM_BINS)
 {
     const int64_t *need = exact ? nullptr : (const int64_t *)(P->bins + BIN_TOTAL_CAP);
-    for (int q = 0; q < P->cfg.nb; q++)
+    for (int q = 0; q < P->cfg.nb && q < nbins; q++)
         launch_bin<SR>(P, q, A, B, M, exact ? P->h_bins[q + 1] : P->m, exact, need, s);
+}
+
+// Do C's rows fit the shared memory of k_saxpy_tile, and B's tile starts a
+// modest array?  (A row of fp64 values up to about 26000 columns; one-row
+// products have their own kernels.)
+template <class SR>
+static bool tile_fits(const SaxpyPlan *P, const DevCSR &A, const DevCSR &B)
+{
+    static const size_t room = [] {
+        cudaFuncAttributes fa;
+        const void *fn = (const void *)k_saxpy_tile<SR>;
+        if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) { cudaGetLastError(); return (size_t)0; }
+        allow_dynamic_smem(fn);
+        return runtime().smem_optin - fa.sharedSizeBytes;
+    }();
+    return A.nrows > 1 && tile_smem<typename SR::z_t>(B.ncols, P->has_mask) + 1024 <= room &&
+           B.nrows * (int64_t)(TILE_T + 1) * 4 <= ((int64_t)256 << 20);
+}
+
+// the rows past the first bin (counts from plan_read) by k_saxpy_tile
+template <class SR>
+static int exec_tile(SaxpyPlan *P, const DevCSR *M, const DevCSR &A, const DevCSR &B,
+                     cudaStream_t s)
+{
+    using Z = typename SR::z_t;
+    const int nb = P->cfg.nb;
+    int n = 0;
+    for (int q = 2; q <= nb + 1; q++) n += P->h_bins[q];
+    if (n == 0) return SUCCESS;
+    int *hist = nullptr, *next = nullptr;
+    int32_t *bound = nullptr, *split = nullptr;
+    Carve cv(s);
+    auto layout = [&]() {
+        next = cv.take<int>(1);
+        hist = cv.take<int>(B.ncols);
+        bound = cv.take<int32_t>(TILE_T + 1);
+        split = cv.take<int32_t>(B.nrows * (TILE_T + 1));
+    };
+    layout();
+    if (!cv.alloc()) return OUT_OF_MEMORY;
+    layout();
+    cudaMemsetAsync(next, 0, (size_t)((char *)(hist + B.ncols) - (char *)next), s);
+    k_tile_hist<<<nblocks(B.nnz, 256, 8), 256, 0, s>>>(B.j, B.nnz, hist);
+    k_tile_bounds<<<1, 1024, 0, s>>>(hist, (int32_t)B.ncols, B.nnz, bound);
+    k_tile_split<<<nblocks(B.nrows * (TILE_T + 1), 256, 16), 256, 0, s>>>(B.p, B.j, B.nrows,
+                                                                         bound, split);
+    const size_t smem = tile_smem<Z>(B.ncols, P->has_mask);
+    int64_t blocks = resident_blocks((const void *)k_saxpy_tile<SR>, TILE_WARPS * 32, smem);
+    if (blocks > n) blocks = n;
+    const int ps = prof_begin("saxpy3_numeric", s);
+    k_saxpy_tile<SR><<<(unsigned)blocks, TILE_WARPS * 32, smem, s>>>(
+        P->bin_rows + P->h_start[2], n, next, esc_in(M, P->mask_comp, A, B), split,
+        (int32_t)B.ncols, P->flops, P->slot_off, P->Tj, (Z *)P->Tx, P->row_cnt);
+    prof_end(ps, s);
+    dfree(cv.base, s);
+    return cuda_to_info(cudaGetLastError());
 }
 
 // the heavy rows (counts from plan_read, accumulators from plan_alloc_heavy)
@@ -2739,8 +3035,11 @@ static int saxpy3_t(DevCSR &C, const DevCSR *M, bool mask_comp, const DevCSR &A,
         T.j = nullptr; T.x = nullptr;
         cap = -1;
     }
+    // rows past the first bin wait for the read where they go to k_saxpy_tile
+    const bool tile = tile_fits<SR>(P, A, B);
+    const int nbins = tile ? 1 : MAX_SMEM_BINS;
     const int ps = prof_begin("saxpy3_numeric", s);
-    exec_light<SR>(P, M, A, B, false, s);
+    exec_light<SR>(P, M, A, B, false, s, nbins);
     prof_end(ps, s);
     exec_counts(P, T.p, nullptr, s);
     if (cap >= 0) exec_pack<Z>(P, T.j, (Z *)T.x, s, cap);
@@ -2752,10 +3051,14 @@ static int saxpy3_t(DevCSR &C, const DevCSR *M, bool mask_comp, const DevCSR &A,
         slots = src.get(slot_bytes(P, P->total_cap + P->total_cap / 4));
         if (!slots) { dev_free(T, s); return OUT_OF_MEMORY; }
         plan_place_slots(P, slots, src.have);
-        exec_light<SR>(P, M, A, B, true, s);
+        exec_light<SR>(P, M, A, B, true, s, nbins);
         again = true;
     }
-    if (P->h_bins[P->cfg.nb + 1] > 0) {
+    if (tile) {
+        for (int q = 2; q <= P->cfg.nb + 1; q++) again |= P->h_bins[q] > 0;
+        info = exec_tile<SR>(P, M, A, B, s);
+        if (info != SUCCESS) { dev_free(T, s); return info; }
+    } else if (P->h_bins[P->cfg.nb + 1] > 0) {
         info = plan_alloc_heavy<SR>(P, s);
         if (info != SUCCESS) { dev_free(T, s); return info; }
         exec_heavy<SR>(P, M, A, B, s);

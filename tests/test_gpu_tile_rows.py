@@ -1,0 +1,64 @@
+"""Rows of more than 256 products: dense in shared memory where C's rows fit
+(k_saxpy_tile), by hash tables and dense rows in global memory where they do
+not.  Both at the edges of their ranges, against the oracle, bit for bit."""
+
+import numpy as np
+import pytest
+
+from graphblas_b200 import workloads as W
+from tests.helpers import assert_exact
+
+pytestmark = pytest.mark.gpu
+
+SEMIRINGS = [("PLUS", "TIMES", "fp64", np.float64), ("PLUS", "TIMES", "fp32", np.float32),
+             ("MIN", "PLUS", "fp32", np.float32), ("PLUS", "PAIR", "int64", np.int64),
+             ("ANY", "SECONDI", "int64", np.int64), ("LOR", "LAND", "bool", np.bool_)]
+
+
+def ragged(nrows, ncols, lengths, seed, dtype, skew):
+    """Rows of the given lengths; with skew the low columns are drawn most."""
+    rng = np.random.default_rng(seed)
+    weight = 1.0 / (np.arange(ncols) + 5.0) if skew else np.ones(ncols)
+    weight /= weight.sum()
+    rows = [np.sort(rng.choice(ncols, min(int(k), ncols), replace=False, p=weight))
+            for k in lengths]
+    p = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int64)
+    i = np.concatenate(rows).astype(np.int64) if p[-1] else np.zeros(0, np.int64)
+    x = rng.random(len(i)) < 0.7 if dtype == np.bool_ else (rng.random(len(i)) * 8 - 4).astype(dtype)
+    return W.Csr(nrows, ncols, p, i, x)
+
+
+# columns of C: one word and its neighbours; a few tiles; B wider than its
+# entries; past what fits in shared memory with 8-byte (30000) and with 4-byte
+# values (60000)
+SHAPES = [(20, 300, 32), (20, 300, 33), (40, 700, 1000), (30, 600, 20000), (25, 500, 30000),
+          (25, 500, 60000)]
+
+
+@pytest.mark.parametrize("add,mult,tname,np_t", SEMIRINGS)
+@pytest.mark.parametrize("mask", [None, "plain", "complement"])
+@pytest.mark.parametrize("m,k,n", SHAPES)
+def test_rows_past_the_first_bin(gpu, oracle, add, mult, tname, np_t, mask, m, k, n):
+    gb = gpu
+    tc = gb.TYPES[tname]
+    rng = np.random.default_rng(5)
+    # rows of A: empty, short, past 32 entries, and every row of B
+    alen = rng.choice([0, 1, 20, 33, 120], m)
+    alen[m // 2] = k
+    A = ragged(m, k, alen, 1, np_t, False)
+    blen = rng.choice([0, 1, 30, 90], k)
+    blen[k // 3] = n
+    B = ragged(k, n, blen, 2, np_t, True)
+    M = ragged(m, n, rng.integers(0, n // 2, m), 3, np.bool_, False) if mask else None
+    if M:
+        M.x = None
+    dA, dB = gb.DMatrix.upload(A, tname), gb.DMatrix.upload(B, tname)
+    dM = gb.DMatrix.upload(M, "bool") if M else None
+    C = gb.saxpy3(dA, dB, gb.semiring(add, mult, tname), M=dM, mask_comp=mask == "complement")
+    got = C.download()
+    want = oracle.saxpy(m, n, (A.p, A.i, A.x, tc), (B.p, B.i, B.x, tc), add, mult, tc,
+                        M=(M.p, M.i, None, 1) if M else None, mask_comp=mask == "complement")
+    assert_exact(got, want, "%s_%s_%s" % (add, mult, tname))
+    for d in (dA, dB, dM, C):
+        if d is not None:
+            d.free()
