@@ -979,13 +979,16 @@ k_saxpy_small(int32_t m, int32_t chunk, EscIn in, long long *__restrict__ part,
 // ---------------------------------------------------------------------------
 
 // One block per row, the row dense in shared memory (a value and a bit per
-// column of C), its columns cut into TILE_T tiles of about as many entries of
-// B each.  A warp takes a few adjacent tiles at a time and streams all of the
-// row's products that fall in them, in ascending k, 32 at a time: no other
-// warp writes those columns, so nothing is synchronised inside the row, the
-// loads of four steps are in flight together, and two products of one column
-// in a step are found by a warp match and folded by the first of them in lane
-// order, which is k order.  Every column is folded in ascending k as in the
+// column of C), its columns cut into a tile of about as many entries of B for
+// each warp.  A warp streams the row's products that fall in its tile, in
+// ascending k, 32 at a time: no other warp writes those columns, so nothing is
+// synchronised inside the row, the loads of four steps are in flight
+// together, and two products of one column in a step are found by a warp
+// match and folded by the first of them in lane order, which is k order.
+// Steps within one row of B need no match (64 cycles of its unit, which
+// bounds the mixed steps); narrower tiles mix more rows and columns meet more
+// often: 32 tiles taken by whichever warp is free took 713 us for the
+// product below.  Every column is folded in ascending k as in the
 // other kernels: the same bits for every semiring.  split[k][t] is where tile
 // t starts in row k of B.
 //
@@ -993,9 +996,9 @@ k_saxpy_small(int32_t m, int32_t chunk, EscIn in, long long *__restrict__ part,
 // synchronisation for each k, and dense rows in global memory by one block
 // with a dependent chain of five loads and a block barrier for each k) were
 // bound by latency: 2509 us for the 38M products (fp64) of the square of a
-// skewed graph of 5000 vertices, against 713 us.
-static constexpr int TILE_T = 32;                // tiles of a row, at most
+// skewed graph of 5000 vertices, against 438 us.
 static constexpr int TILE_WARPS = 8;
+static constexpr int TILE_T = TILE_WARPS;        // tiles of a row
 static constexpr int TILE_U = 4;                 // steps of 32 products in flight
 
 // entries of B in each column
@@ -1065,14 +1068,13 @@ template <class SR>
 __global__ void __launch_bounds__(TILE_WARPS * 32, 4)
 k_saxpy_tile(const int32_t *__restrict__ rows, int nrows, int *__restrict__ next, EscIn in,
              const int32_t *__restrict__ split, int32_t ncols,
-             const int64_t *__restrict__ flops, const int64_t *__restrict__ slot_off,
-             int32_t *__restrict__ Tj, typename SR::z_t *__restrict__ Tx,
+             const int64_t *__restrict__ slot_off, int32_t *__restrict__ Tj, typename SR::z_t *__restrict__ Tx,
              int32_t *__restrict__ row_cnt)
 {
     using Z = typename SR::z_t;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ EscEnt<Z> s_ent[TILE_WARPS][ESC_ENTS];
-    __shared__ int s_row, s_group;
+    __shared__ int s_row;
     __shared__ int s_w[TILE_WARPS];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const unsigned upto = 0xffffffffu >> (31 - lane), below = upto >> 1;
@@ -1083,7 +1085,7 @@ k_saxpy_tile(const int32_t *__restrict__ rows, int nrows, int *__restrict__ next
     EscEnt<Z> *ent = s_ent[w];
     while (true) {
         __syncthreads();
-        if (tid == 0) { s_row = atomicAdd(next, 1); s_group = 0; }
+        if (tid == 0) s_row = atomicAdd(next, 1);
         for (int q = tid; q < words; q += blockDim.x) {
             bits[q] = 0;
             if (in.has_mask) mbits[q] = 0;
@@ -1097,25 +1099,16 @@ k_saxpy_tile(const int32_t *__restrict__ rows, int nrows, int *__restrict__ next
                 atomicOr(&mbits[in.Mj[pm] >> 5], 1u << (in.Mj[pm] & 31));
             __syncthreads();
         }
-        // tiles that a warp takes at a time: a group of a short row holds a
-        // few hundred products too
-        const int64_t f = flops[i];
-        const int gs = f >= 16384 ? 1 : f >= 4096 ? 2 : 4;
-        while (true) {
-            int g = 0;
-            if (lane == 0) g = atomicAdd(&s_group, 1);
-            g = __shfl_sync(0xffffffffu, g, 0);
-            const int t0 = g * gs;
-            if (t0 >= TILE_T) break;
+        {
             for (int32_t c0 = pa0; c0 < pa1; c0 += ESC_ENTS) {
                 const int32_t pa = c0 + lane;
                 int32_t k = 0, b0 = 0, len = 0;
                 Z a = Z();
                 if (pa < pa1) {
                     k = in.Aj[pa];
-                    const int32_t *sp = split + (int64_t)k * (TILE_T + 1) + t0;
+                    const int32_t *sp = split + (int64_t)k * (TILE_T + 1) + w;
                     b0 = sp[0];
-                    len = sp[gs] - b0;
+                    len = sp[1] - b0;
                     if (SR::needs_a) a = ld_val<Z>(in.Ax, pa, in.a_iso);
                 }
                 int incl = len;
@@ -1134,6 +1127,7 @@ k_saxpy_tile(const int32_t *__restrict__ rows, int nrows, int *__restrict__ next
                 for (int q0 = 0; q0 < total; q0 += 32 * TILE_U) {
                     int32_t j[TILE_U];
                     int src[TILE_U];
+                    bool mixed[TILE_U];
                     Z b[TILE_U];
                     #pragma unroll
                     for (int u = 0; u < TILE_U; u++) {
@@ -1142,6 +1136,7 @@ k_saxpy_tile(const int32_t *__restrict__ rows, int nrows, int *__restrict__ next
                                              ? 1u << (excl & 31) : 0u);
                         src[u] = c + __popc(st & upto);
                         c += __popc(st);
+                        mixed[u] = (st & ~1u) != 0;
                         const int q = q0 + u * 32 + lane;
                         j[u] = -1;
                         b[u] = Z();
@@ -1162,8 +1157,9 @@ k_saxpy_tile(const int32_t *__restrict__ rows, int nrows, int *__restrict__ next
                             const EscEnt<Z> e = ent[src[u]];
                             z = SR::F::f(e.a, b[u], i, e.k, j[u]);
                         }
-                        const unsigned same =
-                            __match_any_sync(0xffffffffu, valid ? j[u] : -1 - lane);
+                        unsigned same = 1u << lane;
+                        if (mixed[u])
+                            same = __match_any_sync(0xffffffffu, valid ? j[u] : -1 - lane);
                         const bool first = valid && (same & below) == 0;
                         unsigned rest = first ? same & ~upto : 0u;
                         const Z own = z;
@@ -1172,7 +1168,7 @@ k_saxpy_tile(const int32_t *__restrict__ rows, int nrows, int *__restrict__ next
                             was = (bits[j[u] >> 5] >> (j[u] & 31)) & 1u;
                             if (was) z = SR::M::update(acc[j[u]], z);
                         }
-                        while (__any_sync(0xffffffffu, rest != 0)) {
+                        while (mixed[u] && __any_sync(0xffffffffu, rest != 0)) {
                             const Z t = shfl<Z>(own, rest ? __ffs(rest) - 1 : lane);
                             if (rest) { z = SR::M::update(z, t); rest &= rest - 1; }
                         }
@@ -2657,7 +2653,7 @@ static int exec_tile(SaxpyPlan *P, const DevCSR *M, const DevCSR &A, const DevCS
     const int ps = prof_begin("saxpy3_numeric", s);
     k_saxpy_tile<SR><<<(unsigned)blocks, TILE_WARPS * 32, smem, s>>>(
         P->bin_rows + P->h_start[2], n, next, esc_in(M, P->mask_comp, A, B), split,
-        (int32_t)B.ncols, P->flops, P->slot_off, P->Tj, (Z *)P->Tx, P->row_cnt);
+        (int32_t)B.ncols, P->slot_off, P->Tj, (Z *)P->Tx, P->row_cnt);
     prof_end(ps, s);
     dfree(cv.base, s);
     return cuda_to_info(cudaGetLastError());
@@ -3028,20 +3024,23 @@ static int saxpy3_t(DevCSR &C, const DevCSR *M, bool mask_comp, const DevCSR &A,
     if (cg > cfull + 64.0) cg = cfull + 64.0;
     if (cg > (double)(INT32_MAX - 1)) cg = (double)(INT32_MAX - 1);
     int64_t cap = (int64_t)cg;
-    T.j = (int32_t *)dalloc((size_t)(cap + 1) * 4, s);
-    T.x = dalloc((size_t)(cap + 1) * sizeof(Z), s);
+    // rows past the first bin wait for the read where they go to k_saxpy_tile:
+    // with a mean row past it most do, and C is sized and packed after them
+    const bool tile = tile_fits<SR>(P, A, B);
+    const int nbins = tile ? 1 : MAX_SMEM_BINS;
+    const bool late = tile && cg > 1.15 * (double)P->cfg.bin[0].limit * (double)m;
+    if (late) cap = -1;
+    else T.j = (int32_t *)dalloc((size_t)(cap + 1) * 4, s);
+    if (!late) T.x = dalloc((size_t)(cap + 1) * sizeof(Z), s);
     if (!T.j || !T.x) {
         dfree(T.j, s); dfree(T.x, s);
         T.j = nullptr; T.x = nullptr;
         cap = -1;
     }
-    // rows past the first bin wait for the read where they go to k_saxpy_tile
-    const bool tile = tile_fits<SR>(P, A, B);
-    const int nbins = tile ? 1 : MAX_SMEM_BINS;
     const int ps = prof_begin("saxpy3_numeric", s);
     exec_light<SR>(P, M, A, B, false, s, nbins);
     prof_end(ps, s);
-    exec_counts(P, T.p, nullptr, s);
+    if (!late) exec_counts(P, T.p, nullptr, s);
     if (cap >= 0) exec_pack<Z>(P, T.j, (Z *)T.x, s, cap);
     info = plan_read(P, s);
     if (info != SUCCESS) { dev_free(T, s); return info; }
@@ -3064,7 +3063,7 @@ static int saxpy3_t(DevCSR &C, const DevCSR *M, bool mask_comp, const DevCSR &A,
         exec_heavy<SR>(P, M, A, B, s);
         again = true;
     }
-    if (again) {
+    if (again || late) {
         exec_counts(P, T.p, nullptr, s);
         info = plan_read(P, s);
         if (info != SUCCESS) { dev_free(T, s); return info; }
