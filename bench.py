@@ -204,14 +204,15 @@ class TriCount:
         return n
 
     def launches_per_step(self):
-        # the counting path (masks of 1024+ entries): classify, plan, route,
-        # the warp-hash and block-bitmap count kernels and the merge kernel;
-        # the sum of C comes back with the call, so the reduction launches
-        # nothing.  Smaller masks: classify and intersect, then the two
-        # reduction launches.
+        # the grouped path (masks of 1024+ entries): classify, plan, route
+        # and the warp-hash and block-bitmap count kernels (the merge kernel
+        # only where a row spans more columns than the bitmap holds); the sum
+        # of C comes back with the call, so the reduction launches nothing.
+        # Smaller masks: classify and intersect, then the two reduction
+        # launches.
         if self.L.nnz < 1024:
             return 4
-        return 6
+        return 5
 
     def cpu_baseline(self, R, ncores):
         ntri, times = R.tricount(self.S.nrows, self.L.p, self.L.i, self.U.p, self.U.i, reps=5)

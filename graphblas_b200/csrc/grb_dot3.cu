@@ -390,14 +390,20 @@ static constexpr int CT_BM_THREADS = 1024;
 static constexpr int CT_ITEM_BM = 2048;      // entries per bitmap item, at most
 static constexpr int CT_ITEM_H = 1024;       // entries per hash item, at most
 static constexpr int64_t CT_WORK_BM = 1 << 20;   // probes per bitmap item, about
-static constexpr int64_t CT_WORK_H = 1 << 14;    // probes per hash item, about
+static constexpr int64_t CT_WORK_H = 1 << 14;    // probes per hash item, about, at most
+static constexpr int64_t CT_WORK_H_MIN = 1 << 9; // and at least
 static constexpr int CT_PER_LANE = 16;       // list elements per lane of a lane group
 static constexpr int CT_LONG = 256;          // lists this long go to the front of a bucket
 static constexpr int CT_TILE_T = 256;        // plan: threads per tile
 static constexpr int CT_TILE_K = 8;          // plan: keys per thread
 static constexpr int CT_TILE = CT_TILE_T * CT_TILE_K;
 static constexpr int CT_MERGE = -2;          // queue key of an entry for the merge kernel
+// The grouped path's masks: with fewer than CT_SMALL_COLS columns its five
+// launches only pay from about 128K entries on (triangle counts, two launches
+// of merges against five: 8000 vertices, 113K entries, 141 and 167 us; 16000
+// vertices, 230K entries, 227 and 157 us; 30000 vertices, 416 and 230 us).
 static constexpr int64_t CT_MIN_ENTRIES = 1024;
+static constexpr int64_t CT_SMALL_COLS = 32736, CT_SMALL_ENTRIES = 1 << 17;
 
 // per mask entry: group key (-1: done, CT_MERGE: merge kernel), rank among
 // the group's long (rank >= 0) or short (rank < 0: -rank-1) lists, and the
@@ -508,7 +514,7 @@ __device__ __forceinline__ void ct_key_plan(const int32_t *__restrict__ gcnt,
                                             const unsigned long long *__restrict__ gwork,
                                             int64_t t, int64_t nkeys, int32_t nrows,
                                             const int32_t *__restrict__ Ap,
-                                            const int32_t *__restrict__ Bp,
+                                            const int32_t *__restrict__ Bp, int64_t work_h,
                                             int32_t &c, int32_t &nb, int32_t &nh)
 {
     c = 0; nb = 0; nh = 0;
@@ -519,7 +525,7 @@ __device__ __forceinline__ void ct_key_plan(const int32_t *__restrict__ gcnt,
     const int32_t r = by_row ? (int32_t)t : (int32_t)(t - nrows);
     const int32_t klen = by_row ? Ap[r + 1] - Ap[r] : Bp[r + 1] - Bp[r];
     const bool big = klen > CT_BM_KEY;
-    const int64_t chunk = big ? CT_WORK_BM : CT_WORK_H;
+    const int64_t chunk = big ? CT_WORK_BM : work_h;
     const int32_t emax = big ? CT_ITEM_BM : CT_ITEM_H;
     int64_t n = ((int64_t)gwork[t] + chunk - 1) / chunk;
     const int64_t nmin = (c + emax - 1) / emax, nmax = c / 16 > nmin ? c / 16 : nmin;
@@ -555,7 +561,7 @@ __global__ void __launch_bounds__(CT_TILE_T)
 k_ct_plan(const int32_t *__restrict__ gcnt, const unsigned long long *__restrict__ gwork,
           int64_t nkeys, int32_t nrows,
           const int32_t *__restrict__ Ap, const int32_t *__restrict__ Aj,
-          const int32_t *__restrict__ Bp, const int32_t *__restrict__ Bj,
+          const int32_t *__restrict__ Bp, const int32_t *__restrict__ Bj, int64_t work_h,
           unsigned long long *__restrict__ status, int *__restrict__ tile_ctr,
           int32_t *__restrict__ boff, CtItem *__restrict__ items_bm,
           CtItem *__restrict__ items_h, int32_t *__restrict__ totals)
@@ -573,7 +579,7 @@ k_ct_plan(const int32_t *__restrict__ gcnt, const unsigned long long *__restrict
     #pragma unroll
     for (int k = 0; k < CT_TILE_K; k++) {
         int32_t c, nb, nh;
-        ct_key_plan(gcnt, gwork, t0 + k, nkeys, nrows, Ap, Bp, c, nb, nh);
+        ct_key_plan(gcnt, gwork, t0 + k, nkeys, nrows, Ap, Bp, work_h, c, nb, nh);
         sb += nb; sh += nh; sc += c;
     }
     int ib = sb, ih = sh, ic = sc, tb, th, tc;
@@ -614,7 +620,7 @@ k_ct_plan(const int32_t *__restrict__ gcnt, const unsigned long long *__restrict
     for (int k = 0; k < CT_TILE_K; k++) {
         const int64_t t = t0 + k;
         int32_t c, nb, nh;
-        ct_key_plan(gcnt, gwork, t, nkeys, nrows, Ap, Bp, c, nb, nh);
+        ct_key_plan(gcnt, gwork, t, nkeys, nrows, Ap, Bp, work_h, c, nb, nh);
         if (t < nkeys) boff[t] = (int32_t)oc;
         const int32_t n = nb + nh;
         if (n > 0) {
@@ -1138,7 +1144,7 @@ static uint32_t ct_bitmap_words(int64_t ncols)
     const int64_t need = ((ncols + 31) / 32 + 1 + 3) & ~(int64_t)3;
     const int64_t cap = avail & ~(int64_t)3;
     const int64_t w = need < cap ? need : cap;
-    return w >= 1024 ? (uint32_t)(w - 1) : 0;
+    return w >= 4 ? (uint32_t)(w - 1) : 0;
 }
 
 template <class SR>
@@ -1199,12 +1205,20 @@ static int dot3_count_launch(DevCSR &C, const DevCSR &M, bool mask_struct, const
     const bool vec = ((((uintptr_t)A.j) | ((uintptr_t)B.j)) & 15) == 0;
     int64_t blocks = ((mnz + 31) / 32 + 7) / 8;
     if (blocks > (int64_t)nsm * 16) blocks = (int64_t)nsm * 16;
+    // Hash items: about four for each resident warp, from the mean lists.  An
+    // item is one warp's, so on a small graph items of CT_WORK_H probes leave
+    // most warps idle: 1024 vertices, 67 us of hash kernel so, 18 us with
+    // items of 512; R-MAT 20, 750 us and 708.
+    const double mean = 0.5 * ((double)A.nnz / (double)std::max<int64_t>(A.nrows, 1) +
+                               (double)B.nnz / (double)std::max<int64_t>(B.nrows, 1));
+    int64_t work_h = (int64_t)((double)mnz * mean / (double)(nsm * 5 * CT_H_WARPS * 4));
+    work_h = std::min(std::max(work_h, CT_WORK_H_MIN), CT_WORK_H);
     const int ps = prof_begin("dot3", s);
     k_ct_classify<SR><<<(unsigned)blocks, 256, 0, s>>>(
         M.p, M.j, mask_struct ? nullptr : M.x, M.type, mask_struct, mnz, M.nrows,
         A.p, A.j, B.p, B.j, bm_words * 32u, spans_fit, C.j, queue, gcnt, gwork, zc);
     k_ct_plan<<<(unsigned)ntiles, CT_TILE_T, 0, s>>>(
-        gcnt, gwork, nkeys, (int32_t)M.nrows, A.p, A.j, B.p, B.j, status, tile_ctr, boff,
+        gcnt, gwork, nkeys, (int32_t)M.nrows, A.p, A.j, B.p, B.j, work_h, status, tile_ctr, boff,
         items_bm, items_h, totals);
     k_ct_route<<<(unsigned)blocks, 256, 0, s>>>(queue, mnz, (int32_t)M.nrows, gcnt, boff,
                                                  bucket, M.p, M.j, A.p, B.p, mq, mq_len);
@@ -1214,9 +1228,11 @@ static int dot3_count_launch(DevCSR &C, const DevCSR &M, bool mask_struct, const
     k_ct_bitmap<SR><<<nsm, CT_BM_THREADS, (size_t)(bm_words + 1) * 4, s>>>(
         items_bm, totals, inext_bm, (int32_t)M.nrows, bucket, A.j, B.j, vec,
         bm_words, C.j, (Z *)C.x, sum, zc);
-    k_dot3_intersect<SR><<<nsm * 8, 256, 0, s>>>(
-        mq, nullptr, mq_len, mq_next, A.j, A.x, A.iso, B.j, B.x, B.iso, C.j, (Z *)C.x, zc,
-        sum);
+    // only a row that spans more columns than the bitmap holds is merged
+    if (!spans_fit)
+        k_dot3_intersect<SR><<<nsm * 8, 256, 0, s>>>(
+            mq, nullptr, mq_len, mq_next, A.j, A.x, A.iso, B.j, B.x, B.iso, C.j, (Z *)C.x, zc,
+            sum);
     prof_end(ps, s);
     // the totals, the zombie count and the live sum in one read
     unsigned long long hv[10];
@@ -1236,7 +1252,7 @@ static int dot3_launch(DevCSR &C, const DevCSR &M, bool mask_struct,
     const int64_t mnz = M.nnz;
     C.nrows = M.nrows; C.ncols = M.ncols; C.nnz = mnz; C.type = 0; C.iso = false;
     if constexpr (IsCount<SR>::value) {
-        if (mnz >= CT_MIN_ENTRIES && M.nrows + B.nrows < INT32_MAX) {
+        if (mnz >= (A.ncols < CT_SMALL_COLS ? CT_SMALL_ENTRIES : CT_MIN_ENTRIES) && M.nrows + B.nrows < INT32_MAX) {
             const int info = dot3_count_launch<SR>(C, M, mask_struct, A, B, s, live_sum);
             if (info != NO_VALUE) return info;
         }
