@@ -248,10 +248,8 @@ class Saxpy:
         self.products = int(np.sum(deg[self.A.i]))
         self.flops = 2.0 * self.products
         self.workload = "saxpy3_er16384_d8_plus_times_fp64"
-        # DRAM bytes of the one-launch product kernel per launch (ncu capture
-        # of this workload at this size: the inputs come from L2, the written
-        # slots stay there)
-        self.traffic_per_launch = 3.46e6
+        # not measured for the kernel as it is
+        self.traffic_per_launch = None
 
     def config(self):
         return {"n": self.n, "nnz_A": int(self.A.nnz), "products": self.products,
@@ -377,11 +375,8 @@ class Bfs:
         # writes
         self.alg_bytes = 8.0 * self.n + 4.0 * self.S.nnz + 8.0 * self.n
         self.basis = "S read once (offsets and indices), the parent vector written once"
-        # DRAM bytes of the traversal's numeric launches (one per level): the
-        # dense-row product kernel read and wrote 744 MB over a traversal in
-        # one ncu capture at this size (the dense row itself stays in L2);
-        # the other kernels of the level move little.  Per numeric launch:
-        self.traffic_per_launch = 744e6 / 6 if self.scale == 22 else None
+        # not measured for the kernels as they are
+        self.traffic_per_launch = None
 
     def bfs(self, Sg):
         api = self.api
@@ -441,14 +436,11 @@ class Bfs:
         return self.edges
 
     def launches_per_step(self):
-        # levels whose frontier makes the row heavy go straight to the dense
-        # row: prep, product-index scan, products, compaction, row-offset
-        # scan, pack (6); the first and last levels (small frontiers) take
-        # the binned path first: flop counts, bins, slot scan, bin fill,
-        # three bin kernels, row-offset scan, then the dense row (14); each
-        # parent assign but the last level's is one union launch
+        # a level: the accumulator's prep with the scan of the rows' lengths,
+        # the products, and the compaction (3); each parent assign but the
+        # last level's is one union launch
         lev = max(getattr(self, "levels", 1), 1)
-        return 2 * 14 + 6 * max(lev - 2, 0) + (lev - 1)
+        return 3 * lev + (lev - 1)
 
     def cpu_baseline(self, R, ncores):
         """The reference's traversal on all cores, timed (median of 3), and
@@ -540,14 +532,14 @@ class BfsPushPull(Bfs):
         lev = max(getattr(self, "levels", 1), 1)
         pulls = max(getattr(self, "pull_levels", 0), 0)
         push = lev - pulls
-        return 5 * pulls + 14 * min(push, 2) + 6 * max(push - 2, 0) + (lev - 1)
+        return 5 * pulls + 3 * push + (lev - 1)
 
 
 CONFIGS = {"tc": TriCount, "saxpy": Saxpy, "bfs": Bfs, "bfs_pushpull": BfsPushPull}
 SUB_CONFIGS = ("saxpy", "bfs", "bfs_pushpull", "batch", "serve")
 
 # DRAM bytes (read + write) of one triangle-count dot3 call at R-MAT scale 20,
-# summed over its six kernels from one ncu capture of this workload at this
+# summed over its kernels from one ncu capture of this workload at this
 # size (dram__bytes_read.sum + dram__bytes_write.sum)
 TC_TRAFFIC_RMAT20 = 2.98e9
 

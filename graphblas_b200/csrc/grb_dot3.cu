@@ -23,7 +23,8 @@
 //     heavy entries over every warp of the GPU.
 //
 // Counting semirings (PLUS_PAIR on integers: triangle and support counts)
-// on masks of 65536+ entries take a third route for most queued entries:
+// on masks of 1024+ entries (131072+ with fewer than 32736 columns) take a
+// third route for most queued entries:
 // entries sharing their longer list (row i of A, or row j of B) form a
 // group, the shared row is loaded once into a shared-memory bitmap (key rows
 // over 256 entries, one block per SM) or a per-warp hash table (shorter key

@@ -14,13 +14,18 @@
 //        short rows (<= 256 products by default): one warp expands the row's
 //        products into shared memory, sorts them by (column, position) and
 //        folds equal columns in ascending k (expand-sort-compress);
-//        medium rows: a group of TPR threads owns one row and a
-//        shared-memory open-addressing hash table of CAP slots (the
+//        longer rows, where a row of C fits in shared memory: a block per
+//        row, the row dense, a column tile per warp that streams its products
+//        in ascending k (k_saxpy_tile);
+//        where it does not, medium rows: a group of TPR threads owns one row
+//        and a shared-memory open-addressing hash table of CAP slots (the
 //        reference's coarse hash task, GB_AxB_saxpy3_coarseHash_phase5.c,
 //        with linear probing on GB_HASHF-style keys, math/include/GB_hash.h);
 //        heavy rows: a dense accumulator in global memory (Gustavson,
 //        GB_AxB_saxpy3_coarseGus_*_phase5.c) with block-cooperative, ordered
 //        compaction.
+//      One-row products with order-free monoids (vxm) and products of short
+//      rows skip these phases (k_row_prep, k_saxpy_small).
 //      In every bin the row's k loop runs in ascending k and the threads of
 //      the group split B(k,:), whose column indices are distinct, so every
 //      C(i,j) sees its terms in the reference's order: first term written,
@@ -731,6 +736,8 @@ __device__ __forceinline__ void esc_fold(int n, int heads, int posb, const KT *k
     }
 }
 
+// (60M products of short rows, fp32: 902 us; six blocks an SM spill and take
+// 898.)
 template <class SR, typename KT>
 __global__ void __launch_bounds__(ESC_WARPS * 32, 4)
 k_saxpy_esc(BinRows br, int cap, int posb, EscIn in, const int64_t *__restrict__ slot_off,
@@ -779,10 +786,12 @@ k_saxpy_esc(BinRows br, int cap, int posb, EscIn in, const int64_t *__restrict__
 //
 // Bound by instruction issue and by L2 latency (the gathers of B's rows), so
 // every entry crosses memory once: no slots, and no pass that packs them.
-// 65536 rows of 4-16 entries (6.5M products, fp64): 142 us, where the
+// 65536 rows of 4-16 entries (6.5M products, fp64): 138 us, where the
 // separate flop count, bins, slots, row offsets and pack took 200 us.
-// A 24 KB arena of 512 12-byte products a warp holds four rows of a hundred
-// products, so that a block's look-back is paid once for 32 rows.
+// An arena of 384 12-byte products a warp holds three rows of a hundred, so
+// that a block's look-back is paid once for 24 rows, and leaves room for five
+// blocks an SM (a call 169-171 us; four blocks with 512 products 197, six with
+// 256 171, and the shortest products slower by 2%).
 //
 // No block waits for one that has not started, so the launch needs no
 // co-residency and runs beside other kernels.  tot[1] = 0 (done),
@@ -794,7 +803,7 @@ k_saxpy_esc(BinRows br, int cap, int posb, EscIn in, const int64_t *__restrict__
 static constexpr int SMALL_CAP = 256;              // products per row, at most
 static constexpr int SMALL_POSB = 8;               // log2(SMALL_CAP)
 static constexpr int SMALL_CHUNK = 128;            // rows per block, at most
-static constexpr int SMALL_ARENA = 6144;           // bytes of products a warp holds
+static constexpr int SMALL_ARENA = 4608;           // bytes of products a warp holds
 enum { SMALL_DONE = 0, SMALL_TOO_LONG = 1, SMALL_NO_ROOM = 3 };
 
 template <typename Z> __host__ __device__ constexpr int small_arena_entries()
@@ -834,7 +843,7 @@ __device__ __forceinline__ T small_warp_scan(T *v, int n, int lane)
 }
 
 template <class SR>
-__global__ void __launch_bounds__(ESC_WARPS * 32, 4)
+__global__ void __launch_bounds__(ESC_WARPS * 32, 5)
 k_saxpy_small(int32_t m, int32_t chunk, EscIn in, long long *__restrict__ part,
               int32_t *__restrict__ Sj, typename SR::z_t *__restrict__ Sx, int64_t scap,
               int32_t *__restrict__ Cp, int32_t *__restrict__ Cj,
@@ -2156,17 +2165,32 @@ k_pack(int64_t nrows, int span, const int64_t *__restrict__ slot_off,
          s0 < nnz; s0 += nw * span) {
         int64_t r0 = warp_last_le<int64_t, int64_t>(Cp64, nrows, s0, lane);
         const int64_t s1 = s0 + span < nnz ? s0 + span : nnz;
-        for (int64_t base = s0; base < s1; base += 32) {
-            const int64_t e = base + lane;
+        for (int64_t base = s0; base < s1; base += 64) {
+            // two steps at a time, so that both copies are in flight (rows of
+            // 36, 60M entries: 266 us a step at a time, 220 us so).  A walk to
+            // the row: a search of the next 32 row starts took 369 us.
+            const int64_t e = base + lane, e2 = e + 32;
             int64_t r = r0;
-            if (e < s1) {
-                // a walk: C's rows are long (36 entries a row, 60M entries:
-                // 266 us; a search of the next 32 row starts, 369 us)
+            if (e < s1)
                 while (Cp64[r + 1] <= e) r++;
+            int64_t r2 = __shfl_sync(0xffffffffu, r, 31);
+            if (e2 < s1)
+                while (Cp64[r2 + 1] <= e2) r2++;
+            int32_t j = 0, j2 = 0;
+            Z x = Z(), x2 = Z();
+            if (e < s1) {
                 const int64_t src = slot_off[r] + (e - Cp64[r]);
-                Cj[e] = Tj[src];
-                Cx[e] = Tx[src];
+                j = Tj[src];
+                x = Tx[src];
             }
+            if (e2 < s1) {
+                const int64_t src = slot_off[r2] + (e2 - Cp64[r2]);
+                j2 = Tj[src];
+                x2 = Tx[src];
+            }
+            if (e < s1) { Cj[e] = j; Cx[e] = x; }
+            if (e2 < s1) { Cj[e2] = j2; Cx[e2] = x2; }
+            r = r2;
             r0 = __shfl_sync(0xffffffffu, r, 31);
         }
     }
@@ -2906,15 +2930,12 @@ static int saxpy3_row(DevCSR &C, const DevCSR *M, bool mask_comp, const DevCSR &
 // and the output size; only if the slots did not fit (the buffer then grows
 // and the bins run again), heavy rows need their accumulators sized, or C
 // needs larger arrays does more work follow the read.
-// The one-launch path (k_saxpy_small) for products of SMALL_MIN_ROWS to
-// SMALL_MAX_ROWS rows whose rows are expected to fit the expand-sort-compress
-// bin (A's entries times B's mean row length, per row, at most half the
-// bin), with fewer than 2^24 columns (32-bit sort keys).  The slots take
-// SMALL_CAP entries a row from the stream's buffer; C's arrays are sized
-// from B's mean row length as in the general path.  NO_VALUE when the
-// product is not taken, or when the launch found a row past the bin or too
-// little room in C (the caller then runs the general path).
-
+// The one-launch path (k_saxpy_small) for products whose rows are expected to
+// fit the expand-sort-compress bin (A's entries times B's mean row length, per
+// row, at most half the bin), with fewer than 2^24 columns (32-bit sort keys).
+// C's arrays are sized from B's mean row length as in the general path.
+// NO_VALUE when the product is not taken, or when the launch found a row past
+// the bin or too little room in C (the caller then runs the general path).
 template <class SR>
 static int saxpy3_small(DevCSR &C, const DevCSR *M, bool mask_comp, const DevCSR &A,
                         const DevCSR &B, SemiringCode sr, cudaStream_t s)
@@ -2979,7 +3000,8 @@ static int saxpy3_t(DevCSR &C, const DevCSR *M, bool mask_comp, const DevCSR &A,
     if constexpr (SR::order_free) {
         const double est = (double)A.nnz * mean_b;
         const SaxpyConfig dc = saxpy_default_config();
-        const double words = (double)B.ncols * (1.0 + sizeof(typename RowAcc<SR>::W));
+        const double words = (double)B.ncols * ((RowAcc<SR>::flags(M != nullptr) ? 1.0 : 0.0) +
+                                                sizeof(typename RowAcc<SR>::W));
         if (m == 1 && A.nnz > 0 && B.ncols > 0 && words <= (double)((int64_t)4 << 30) &&
             (words <= (double)ROW_CLEAR ||
              est >= 2.0 * (double)dc.bin[dc.nb - 1].limit)) {
